@@ -54,6 +54,32 @@ def test_quantizer_matches_oracle_at_config_sizes(dtype, shape):
     assert torch.equal(packed, torch.from_numpy(w8.c_b200_pack_int8(qo)))
 
 
+@pytest.mark.parametrize("variant", [0, 1])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("K", [64, 128, 192, 320])
+def test_quantizer_at_rounding_boundaries(K, dtype, variant):
+    """Quotients on, just below and just above every half-integer, scales at the ends of the range and beyond it
+    (denormal, zero, huge, infinite), NaN: bit for bit what the division gives, for odd and even numbers of row tiles."""
+    from eet_b200 import EET
+    gen = torch.Generator().manual_seed(K)
+    N = 128
+    w = (torch.randint(-256, 257, (K, N), generator=gen) * 0.5)
+    w[0] = torch.where(torch.arange(N) % 2 == 0, 128.0, -128.0)
+    w = w.to(dtype)
+    ulps = torch.randint(-2, 3, (K, N), generator=gen).to(torch.int16 if dtype == torch.float16 else torch.int32)
+    w[1:] = (w[1:].view(ulps.dtype) + ulps[1:]).view(dtype)
+    expo = torch.linspace(-14 if dtype == torch.float16 else -120, 8 if dtype == torch.float16 else 110, N).round()
+    w = (w.double() * torch.pow(torch.tensor(2.0, dtype=torch.float64), expo)).to(dtype)
+    w[:, 3] = 0.0
+    w[2, 5], w[3, 7], w[4, 9] = float("nan"), float("inf"), float("-inf")
+    w[:, 11] = torch.finfo(dtype).tiny / 4
+    q, packed, scales = EET.quant_weights(w, torch.int8, True, variant=variant)
+    qo, so = w8.c_symmetric_quantize_int8(w.numpy(), variant=variant)
+    assert torch.equal(q, torch.from_numpy(qo))
+    assert torch.equal(_bits(scales), _bits(torch.from_numpy(so)))
+    assert torch.equal(packed, torch.from_numpy(w8.c_b200_pack_int8(qo)))
+
+
 def test_variant_127_and_three_d_input():
     from eet_b200 import EET
     gen = torch.Generator().manual_seed(4)
