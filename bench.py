@@ -183,8 +183,18 @@ def rewind(model, step):
             layer.attention.sync_device_step()
 
 
-def kernel_launches_per_step(n_layers, batch, world):
+def launches_per_step(n_layers, batch, world):
     """Launches of this library's kernels in one decode step (NCCL and torch kernels are not counted)."""
+    if batch <= 16 and world == 1:
+        # per layer: qkv gemm (norm inside), decode attention, out gemm, gate+up gemm (norm and activation inside), down
+        # gemm; per step: advance_steps, embedding gather, first and final rmsnorm, lm_head
+        return 5 * n_layers + 4 + (2 if LM_HEAD_INT8 else 1)
+    return kernel_launches_per_step(n_layers, batch, world)
+
+
+def kernel_launches_per_step(n_layers, batch, world):
+    """The same where the projections leave their epilogues to the kernels behind them (more than 16 rows, or several
+    ranks)."""
     head = 2 if LM_HEAD_INT8 else 1   # int8: lm_head GEMM + fused argmax; fp16: argmax (the GEMM is cuBLAS, not counted)
     if batch <= 64:
         # per layer: rmsnorm(+finalize), qkv gemm, decode attention, out gemm, rmsnorm(+finalize), gate+up gemm,
@@ -218,8 +228,8 @@ def _time_graph(fn, iters_in_graph, reps=5):
 
 
 def time_gemm_shapes(model, batch):
-    """Times the skinny GEMM kernel alone (the accumulate kernel, without the epilogue that the next kernel
-    of a decode step performs) on the real weights of the model: for each of the five projection shapes, all
+    """Times the decode GEMM kernel alone (up to 16 rows the row kernel; above, and per rank, the accumulate kernel,
+    without the epilogue that the next kernel of a decode step performs) on the real weights of the model: for each of the five projection shapes, all
     layers' launches back to back inside one CUDA graph between two CUDA events (one distinct weight buffer
     per layer, GBs in total, so nothing is served from L2).  Returns per-shape results."""
     from eet_b200 import EET
@@ -232,10 +242,15 @@ def time_gemm_shapes(model, batch):
         K, N = getattr(layers[0], wn).shape
         x = torch.randn(batch, K, device=dev).half()
         sums = torch.zeros(batch, N, device=dev, dtype=torch.float32)
+        out = torch.empty(batch, N, device=dev, dtype=torch.float16)
+        row = batch <= 16 and model.model.desc.tp is None
 
         def run():
             for layer in layers:
-                EET.gemm_w8a16_accum(x, getattr(layer, wn), sums)
+                if row:
+                    EET.gemm_w8a16(x, getattr(layer, wn), getattr(layer, sn), out=out)
+                else:
+                    EET.gemm_w8a16_accum(x, getattr(layer, wn), sums)
 
         t = _time_graph(run, len(layers))
         nbytes = N * K + 2 * N + 2 * batch * K + 2 * batch * N
@@ -250,11 +265,12 @@ def skinny_steady_state(device, batch, hbm_peak):
     K, N, M = 8192, 22016, min(batch, 8)
     ws = [torch.randint(-128, 128, (K, N), dtype=torch.int8, device=device) for _ in range(3)]
     x = torch.randn(M, K, device=device).half()
-    sums = torch.zeros(M, N, device=device, dtype=torch.float32)
+    scale = torch.full((N,), 1e-3, device=device).half()
+    out = torch.empty(M, N, device=device, dtype=torch.float16)
 
     def run():
         for i in range(12):
-            EET.gemm_w8a16_accum(x, ws[i % 3], sums)
+            EET.gemm_w8a16(x, ws[i % 3], scale, out=out)
 
     t = _time_graph(run, 12)
     nbytes = N * K + 2 * N + 2 * M * K + 2 * M * N
@@ -604,10 +620,11 @@ def run_ours(args):
                     "consistent": t_e2e >= t_dev * 0.98},
             "prefill": None if prefill_ms is None else {"ms": round(prefill_ms, 2), "tokens": BATCH * PROMPT,
                                                          "tokens_per_s": round(BATCH * PROMPT / prefill_ms * 1e3)},
-            "gpu_launches": kernel_launches_per_step(n_layers, BATCH, world) * K,
+            "gpu_launches": launches_per_step(n_layers, BATCH, world) * K,
             "clocks": clk.summary(), "clocks_e2e": clk_e2e.summary(), "device_status": status,
             "roofline": {"bound": "hbm",
-                         "kernel": f"gemm_skinny_kernel<{1 if BATCH <= 8 else 2}>, fused QKV projection "
+                         "kernel": ("gemm_row_kernel" if BATCH <= 16 and world == 1 else "accumulate kernel") +
+                                   f", fused QKV projection "
                                    f"K={dom['K']} N={dom['N']} M={BATCH}",
                          "achieved": round(dom["gbs"], 1), "peak": pk["hbm_gbs"], "unit": "GB/s",
                          "frac": round(dom["gbs"] / pk["hbm_gbs"], 4), "peak_source": pk["source"],

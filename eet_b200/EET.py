@@ -256,6 +256,20 @@ def gemm_w8a16(x, packed_w, scale, out=None, residual=None, gate=None):
     return out
 
 
+_ROW_MAX_M = 16   # rows of the decode GEMM that finishes its product itself
+
+
+def _gemm_row(x, w, scale, out, M, w2=None, scale2=None, residual=None, norm=None, squares_out=None):
+    """The decode GEMM (M <= 16) with its surroundings in one launch: out = x' @ dequant(w) (+ residual), or
+    gated_silu(x' @ dequant(w), x' @ dequant(w2)), where x' = x, or rmsnorm(x) with norm = (gamma, squares, eps);
+    `squares_out` receives the sums of squares a later call's `norm` needs."""
+    K, N = w.shape
+    gamma, squares, eps = norm if norm is not None else (None, None, 0.0)
+    check(lib.eet_gemm_w8a16_row(x.data_ptr(), _ptr(gamma), _ptr(squares), eps, w.data_ptr(), scale.data_ptr(), _ptr(w2),
+                                 _ptr(scale2), _ptr(residual), out.data_ptr(), _ptr(squares_out), M, N, K, _stream()))
+    return out
+
+
 def _linear(x, w, scale, out, residual=None):
     """One projection of an op: W8A16 when w is int8 (packed), else the fp16 twin - w fp16 [K, N] row-major
     through cuBLAS, as the reference's is_int8 == false branches do (cublasGemmEx in
@@ -316,10 +330,43 @@ class _Pending:
         self.sums, self.scale, self.residual, self.out, self.peer = sums, scale, residual, out, peer
 
 
+class _Squares:
+    """Sums of squares of the 64-channel pieces of an op's (finished) output: the next op of this module that receives
+    the tensor normalises it while its first projection loads it."""
+    __slots__ = ("squares",)
+
+    def __init__(self, squares):
+        self.squares = squares
+
+
 _pending = {}
 _defer = [False]
 _DECODE_MAX_M = 64       # below the tensor-core GEMM's first M
 _DECODE_MAX_M_TP = 64    # rows of the tensor-parallel peer buffers (tp.PeerBuffers.ROWS)
+
+
+def _row_chain(M, desc):
+    """Whether an op called with M rows is part of a chain of this module's ops whose projections finish themselves and
+    whose norms ride on the projections behind them (one GPU, M <= 16)."""
+    return _defer[0] and desc.is_int8 and M <= _ROW_MAX_M and (desc.tp is None or desc.tp.size == 1)
+
+
+def _project_row(x, w, scale, out, residual, M, desc, name):
+    """An op's last projection in such a chain: out = x @ dequant(w) + residual, and its sums of squares for whoever
+    reads `out` next."""
+    N = w.shape[1]
+    squares = _pool.get("squares:" + name, _ROW_MAX_M * (N // 64), torch.float32, desc.device)
+    _gemm_row(x, w, scale, out, M, residual=residual, squares_out=squares)
+    _pending[out.data_ptr()] = _Squares(squares)
+
+
+def _take_squares(x2d, gamma, desc):
+    """The `norm` argument of _gemm_row for an input that such a chain has produced, else None."""
+    p = _pending.get(x2d.data_ptr())
+    if not isinstance(p, _Squares) or not _row_chain(x2d.shape[0], desc):
+        return None
+    del _pending[x2d.data_ptr()]
+    return gamma, p.squares, desc.layernorm_eps
 
 
 def _defer_ok(M, desc):
@@ -327,7 +374,9 @@ def _defer_ok(M, desc):
     if not (_defer[0] and desc.is_int8):
         return False
     tp = desc.tp
-    return M <= (_DECODE_MAX_M_TP if tp is not None and tp.size > 1 else _DECODE_MAX_M)
+    if tp is not None and tp.size > 1:
+        return M <= _DECODE_MAX_M_TP
+    return _ROW_MAX_M < M <= _DECODE_MAX_M
 
 
 class deferred_epilogue:
@@ -350,6 +399,8 @@ class deferred_epilogue:
 
 def flush_pending():
     for p in list(_pending.values()):
+        if isinstance(p, _Squares):
+            continue   # nothing is unfinished
         M, N = p.sums.shape
         if p.peer is not None:
             p.peer[0].tp.all_reduce(p.sums)   # not consumed by an op of this module: plain NCCL path
@@ -362,6 +413,8 @@ def _norm_head(x2d, gamma, eps, xn):
     """RMSNorm at the head of a block; completes x first when it is a deferred output of the previous block."""
     M, n = x2d.shape
     p = _pending.pop(x2d.data_ptr(), None)
+    if isinstance(p, _Squares):
+        p = None
     if p is not None and p.peer is not None:
         pb, which = p.peer
         check(lib.eet_rmsnorm_finalize_tp(p.sums.data_ptr(), pb.inbox_ptrs, pb.tp.size, pb.tp.rank, which,
@@ -485,7 +538,10 @@ class _MmhaBase:
         out = _pool.get("self_mask_attn_cache", d.batch_size * d.max_seq_len * d.hidden_units, torch.float16, d.device)
         out = out[: B * S * d.hidden_units].view(B * S, d.hidden_units)
         inp2d = inp.reshape(B * S, d.hidden_units)
-        if _defer_ok(B * S, d):
+        _pending.pop(out.data_ptr(), None)   # whatever this buffer held before is gone
+        if _row_chain(B * S, d):
+            _project_row(ctx2d, self.out_w, self.out_s, out, inp2d, B * S, d, "self_mask_attn_cache")
+        elif _defer_ok(B * S, d):
             peer = None
             if d.tp is not None and d.tp.size > 1:
                 # row-parallel: the ranks' fp32 partial sums are added before scale, residual and rounding -
@@ -566,10 +622,17 @@ class _MmhaBase:
         if self.step_ > d.max_full_seq_len:
             raise RuntimeError("Exceed the maximum step length")
         H, D = d.head_num, self.size_per_head
-        xn = _pool.get("layernorm_inc", d.batch_size * h, torch.float16, d.device)[: B * h].view(B, h)
-        _norm_head(inp.view(B, h), self.ln_w, d.layernorm_eps, xn)
+        x2d = inp.view(B, h)
         qkv, qkv_sums = None, None
-        if _defer_ok(B, d):
+        norm = _take_squares(x2d, self.ln_w, d)
+        if norm is None:
+            xn = _pool.get("layernorm_inc", d.batch_size * h, torch.float16, d.device)[: B * h].view(B, h)
+            _norm_head(x2d, self.ln_w, d.layernorm_eps, xn)
+        if norm is not None:
+            qkv = _pool.get("qkv_inc", d.batch_size * 3 * self.inner_dim, torch.float16, d.device)
+            qkv = qkv[: B * 3 * self.inner_dim].view(B, 3 * self.inner_dim)
+            _gemm_row(x2d, self.qkv_w, self.qkv_s, qkv, B, norm=norm)
+        elif _defer_ok(B, d):
             # the attention kernel finishes the projection itself: fp16(sums * scale)
             qkv_sums = _pool.zeros("qkv_sums", d.batch_size * 3 * self.inner_dim, torch.float32, d.device)
             qkv_sums = qkv_sums[: B * 3 * self.inner_dim].view(B, 3 * self.inner_dim)
@@ -686,11 +749,15 @@ class GatedFeedForwardNetworkInt8:
         M = B * S
         cap = d.batch_size * d.max_seq_len
         with torch.cuda.device(d.device):
-            xn = _pool.get("layernorm_tensor", cap * h, torch.float16, d.device)[: M * h].view(M, h)
-            _norm_head(input.view(M, h), self.ln_w, d.layernorm_eps, xn)
+            x2d = input.view(M, h)
+            norm = _take_squares(x2d, self.ln_w, d)
+            if norm is None:
+                xn = _pool.get("layernorm_tensor", cap * h, torch.float16, d.device)[: M * h].view(M, h)
+                _norm_head(x2d, self.ln_w, d.layernorm_eps, xn)
             act = _pool.get("ffn_inner_act", cap * self.d_ff, torch.float16, d.device)[: M * self.d_ff].view(M, self.d_ff)
             out = _pool.get(self.cache_name, cap * h, torch.float16, d.device)[: M * h].view(M, h)
-            inp2d = input.view(M, h)
+            inp2d = x2d
+            _pending.pop(out.data_ptr(), None)   # whatever this buffer held before is gone
             deferred = _defer_ok(M, d)
             if deferred:
                 # gate and up in one launch, their epilogues inside the SwiGLU kernel
@@ -699,6 +766,9 @@ class GatedFeedForwardNetworkInt8:
                 gemm_w8a16_accum(xn, self.w0, gs, self.w1, us)
                 check(lib.eet_swiglu_finalize(gs.data_ptr(), self.s0.data_ptr(), us.data_ptr(), self.s1.data_ptr(),
                                               act.data_ptr(), M, self.d_ff, _stream()))
+            elif self.w1.dtype == torch.int8 and M <= _ROW_MAX_M:
+                # norm, gate, up and activation in one launch (the norm on its own where nobody left its squares)
+                _gemm_row(x2d if norm is not None else xn, self.w0, self.s0, act, M, self.w1, self.s1, norm=norm)
             else:
                 _linear(xn, self.w0, self.s0, act)
                 if self.w1.dtype == torch.int8:
@@ -708,7 +778,9 @@ class GatedFeedForwardNetworkInt8:
                     lin = _pool.get("ffn_inner_linear", cap * self.d_ff, torch.float16, d.device)[: M * self.d_ff].view(M, self.d_ff)
                     _linear(xn, self.w1, self.s1, lin)
                     check(lib.eet_swiglu(act.data_ptr(), lin.data_ptr(), M, self.d_ff, _stream()))
-            if deferred and add_residual:
+            if add_residual and _row_chain(M, d):
+                _project_row(act, self.w_out, self.s_out, out, inp2d, M, d, self.cache_name)
+            elif deferred and add_residual:
                 peer = None
                 if d.tp is not None and d.tp.size > 1:
                     pb = d.tp.peer_buffers(h, d.device)   # row-parallel partial sums, see LlamaMmha._project

@@ -46,6 +46,7 @@ static inline bool aligned16(const void* p)
 
 #include "attention.cu"
 #include "gemm_skinny.cu"
+#include "gemm_row.cu"
 #include "gemm_tc.cu"
 #include "gemm_mid.cu"
 #include "attention_tc.cu"
@@ -214,6 +215,23 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
               "eet_gemm_w8a16: epilogues 1 and 2 need a 16-byte aligned second operand");
     const __half* res = epilogue != 0 ? (const __half*)residual : nullptr;
     const int gate = epilogue == 2 ? 1 : 0;
+    if (M <= kRowMaxM) {
+        // decode regime: one launch, no scratch (the check stays: this entry point has always asked for it)
+        EET_CHECK(ws && aligned16(ws) && ws_bytes >= eet_gemm_w8a16_workspace_bytes(M, N, K),
+                  "eet_gemm_w8a16: workspace of %zu bytes is smaller than the %zu needed", ws_bytes,
+                  eet_gemm_w8a16_workspace_bytes(M, N, K));
+        RowGemmArgs r = {};
+        r.A = (const __half*)A;
+        r.B = (const uint8_t*)packedB;
+        r.scale = (const __half*)scale;
+        r.residual = res;
+        r.C = (__half*)C;
+        r.M = M;
+        r.N = N;
+        r.K = K;
+        r.gate = gate;
+        return launch_gemm_row(r, (cudaStream_t)stream);
+    }
     // Above 64 tokens a shape that the 256 x 256 kernel can spread over the machine (plain tiles or split-K
     // clusters) goes there: one launch, epilogue fused, no fp32 scratch.
     const bool tiles_first = M > 64 && gemm_tc_supported(M, N, K) && tc2_split(M, N, K) > 0;
@@ -254,6 +272,37 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
             return rc;
     }
     return 0;
+}
+
+int eet_gemm_w8a16_row(const void* A, const void* gamma, const float* squares_in, float eps, const void* packedB,
+                       const void* scale, const void* packedB2, const void* scale2, const void* residual, void* C,
+                       float* squares_out, int M, int N, int K, void* stream)
+{
+    if (check_gemm("eet_gemm_w8a16_row", A, packedB, M, N, K)) return 1;
+    EET_CHECK(M <= kRowMaxM, "eet_gemm_w8a16_row: M=%d exceeds %d", M, kRowMaxM);
+    if (M == 0) return 0;
+    EET_CHECK(scale && C && aligned16(scale) && aligned16(C) && aligned16(packedB2) && aligned16(scale2) && aligned16(residual) &&
+                  aligned16(gamma),
+              "eet_gemm_w8a16_row: weights, scales, residual, gamma and C must be 16-byte aligned buffers");
+    EET_CHECK((packedB2 == nullptr) == (scale2 == nullptr), "eet_gemm_w8a16_row: B2 and scale2 go together");
+    EET_CHECK((gamma == nullptr) == (squares_in == nullptr), "eet_gemm_w8a16_row: gamma and squares_in go together");
+    EET_CHECK(packedB2 == nullptr || residual == nullptr, "eet_gemm_w8a16_row: a gated product takes no residual");
+    RowGemmArgs r = {};
+    r.A = (const __half*)A;
+    r.B = (const uint8_t*)packedB;
+    r.B2 = (const uint8_t*)packedB2;
+    r.scale = (const __half*)scale;
+    r.scale2 = (const __half*)scale2;
+    r.residual = (const __half*)residual;
+    r.C = (__half*)C;
+    r.gamma = (const __half*)gamma;
+    r.squares_in = squares_in;
+    r.squares_out = squares_out;
+    r.eps = eps;
+    r.M = M;
+    r.N = N;
+    r.K = K;
+    return launch_gemm_row(r, (cudaStream_t)stream);
 }
 
 int eet_gemm_w8a16_noalloc(const void* A, const void* packedB, const void* scale, void* C, int M, int N, int K,

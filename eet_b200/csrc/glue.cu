@@ -15,20 +15,25 @@ namespace {
 
 // y = x * rsqrt(mean(x^2) + eps) * gamma, fp32 math, one fp16 rounding.
 // Reference: T5norm1_kernel_opt<half> (csrc/core/layer_norm.cu:490-531).  One CTA per row; the row is
-// kept in registers between the two phases (n <= 8 * 2 * blockDim).
+// kept in registers between the two phases (n <= 8 * 2 * blockDim).  In a decode step the kernel is nothing but latency:
+// the norm weights are fetched while the preceding kernel still runs, and every warp adds the per-warp sums itself (the
+// same order everywhere), which saves the second block barrier.
 __global__ void __launch_bounds__(1024)
 rmsnorm_kernel(const __half* __restrict__ x, const __half* __restrict__ gamma, __half* __restrict__ y, int n, float eps)
 {
     __shared__ float red[32];
-    __shared__ float s_inv;
     pdl_launch_dependents();
-    pdl_wait();
     const int row = blockIdx.x;
     const int nv = n >> 3;
     const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * n);
-    const uint4* g4 = reinterpret_cast<const uint4*>(gamma);
     uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * n);
-    uint4 v[2];
+    uint4 v[2], g[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i < nv) g[j] = reinterpret_cast<const uint4*>(gamma)[i];
+    }
+    pdl_wait();
     float ss = 0.f;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
@@ -46,20 +51,15 @@ rmsnorm_kernel(const __half* __restrict__ x, const __half* __restrict__ gamma, _
     ss = warp_sum(ss);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        float t = (threadIdx.x < (blockDim.x >> 5)) ? red[threadIdx.x] : 0.f;
-        t = warp_sum(t);
-        if (threadIdx.x == 0) s_inv = rsqrtf(t / n + eps);
-    }
-    __syncthreads();
-    const float inv = s_inv;
+    float t = (threadIdx.x & 31) < (blockDim.x >> 5) ? red[threadIdx.x & 31] : 0.f;
+    t = warp_sum(t);
+    const float inv = rsqrtf(t / n + eps);
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
         const int i = threadIdx.x + j * blockDim.x;
         if (i < nv) {
-            const uint4 g = g4[i];
             const __half2* h = reinterpret_cast<const __half2*>(&v[j]);
-            const __half2* gh = reinterpret_cast<const __half2*>(&g);
+            const __half2* gh = reinterpret_cast<const __half2*>(&g[j]);
             uint4 o;
             __half2* oh = reinterpret_cast<__half2*>(&o);
 #pragma unroll

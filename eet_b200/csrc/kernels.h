@@ -28,6 +28,26 @@ struct GemmArgs {
 size_t skinny_sum_bytes(int M, int N);
 int launch_gemm_skinny(const GemmArgs& a, cudaStream_t stream);
 
+// gemm_row.cu: M <= 16, finished in one launch
+constexpr int kRowMaxM = 16;
+constexpr int kRowMaxSplits = 8;
+struct RowGemmArgs {
+    const __half* A;         // [M][K]
+    const uint8_t* B;        // W8T64
+    const uint8_t* B2;       // null, or a second weight of the same shape: C = gated_silu(A.B, A.B2)
+    const __half* scale;     // [N]
+    const __half* scale2;    // [N], with B2
+    const __half* residual;  // null, or [M][N]: C = A.B + residual, with `gate` C = gated_silu(residual, A.B)
+    __half* C;               // [M][N]
+    const __half* gamma;       // null, or [K]: the activations are rmsnorm(A) with these weights, from ...
+    const float* squares_in;   // ... [M][K/64] sums of squares of A's 64-channel pieces
+    float* squares_out;        // null, or [M][N/64]: the same of C
+    float eps;
+    int M, N, K, gate;
+    int splits;              // CTAs per tile row, chosen by the launcher
+};
+int launch_gemm_row(RowGemmArgs a, cudaStream_t stream);
+
 // gemm_tc.cu (tcgen05 / TMEM)
 bool gemm_tc_supported(int M, int N, int K);
 int tc2_split(int M, int N, int K);  // 0: the 256 x 256 kernel does not take this shape; else its split-K cluster size

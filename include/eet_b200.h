@@ -107,13 +107,27 @@ size_t eet_gemm_w8a16_workspace_bytes(int M, int N, int K);
  *             called from csrc/op/gated_ffn_int8.cpp:290-301) fused in, with its mix of fp32 and fp16 arithmetic.
  *   residual  device fp16 [M][N] for epilogues 1 and 2, else NULL (may alias C)
  * M may be any value >= 0; K and N must be multiples of 64; pointers 16-byte aligned.
- * Kernels: M <= 16 TMA-staged skinny kernel; 16 < M <= 512 (N % 128 == 0) stream-K tcgen05 kernel; above
+ * Kernels: M <= 16 TMA-staged row kernel (one launch, leaves the scratch alone); 16 < M <= 512 (N % 128 == 0) stream-K tcgen05 kernel; above
  * that - and from M = 65 on for shapes (N % 256 == 0) whose 256 x 256 tiles, whole or with their k-blocks split
  * over clusters of 2-4 CTAs, can occupy most of the GPU - tcgen05 kernels with 256 x 256 or 128 x 256 output
  * tiles that need no scratch; shapes none of them takes fall back to the skinny kernel in groups of 128 rows.
  */
 int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* C, int M, int N, int K,
                    const void* residual, int epilogue, void* ws, size_t ws_bytes, void* stream);
+
+/*
+ * The decode GEMM (M <= 16) with what stands around it in a decoder layer, in one launch and without scratch:
+ *   gamma, squares_in  both NULL: the activations are A; else they are rmsnorm(A) with weights gamma [K] and eps, the
+ *                      norm at the head of a block (csrc/core/layer_norm.cu:490-531); squares_in [M][K/64] fp32 holds
+ *                      the sums of squares of A's 64-channel pieces, as the launch that stored A left them:
+ *   squares_out        NULL, or [M][N/64] fp32: the sums of squares of C's 64-channel pieces
+ *   packedB2, scale2   both NULL: C = x.B (+ residual, fp16 add; may be NULL or alias C); else a second weight of the
+ *                      same shape: C = gated_silu(fp16(x.B), fp16(x.B2)), the first half of a gated FFN
+ *                      (csrc/op/gated_ffn_int8.cpp:253-301: two GEMMs and the activation kernel); residual NULL
+ */
+int eet_gemm_w8a16_row(const void* A, const void* gamma, const float* squares_in, float eps, const void* packedB,
+                       const void* scale, const void* packedB2, const void* scale2, const void* residual, void* C,
+                       float* squares_out, int M, int N, int K, void* stream);
 
 /*
  * The two halves of eet_gemm_w8a16 for M <= 512 (the decode regime and small prefills), exposed so that the

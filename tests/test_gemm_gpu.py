@@ -110,6 +110,69 @@ def test_empty_and_invalid():
     assert rc != 0
 
 
+@pytest.mark.parametrize("kind", ["plain", "residual", "gate", "gated", "norm", "norm_gated"])
+@pytest.mark.parametrize("K,N,M", [(64, 64, 1), (512, 128, 16), (1088, 64, 9), (1088, 2560, 8), (4096, 4096, 7), (5120, 5120, 3),
+                                   (2048, 8192, 13), (5120, 13696, 12), (64, 65536, 2)])
+def test_decode_gemm_finished_in_one_launch(K, N, M, kind):
+    """Every cluster size (8, 4, 3, 2, 1), fewer tiles than warps, shares that do not divide, both token groups, each
+    epilogue; the same bits twice (fixed order of the sums).  Bound: fp32 sums, so one fp16 rounding of the product and
+    one of the sum with the residual, 2^-11 each, doubled; the activation's error is its operands' plus its own three
+    fp16 steps.  With the norm inside, the sums of squares come from a call that stores the input (a product with a
+    residual, as in a decoder layer); the activations are rounded once to fp16, at another place than rmsnorm_kernel
+    rounds them: 2^-11 each way and each, over the root of the reduction's length."""
+    from eet_b200 import EET, _lib
+    from eet_b200._lib import check, lib
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    w = [torch.randint(-127, 128, (K, N), generator=gen, device="cuda", dtype=torch.int8) for _ in range(2)]
+    s = [((torch.rand(N, generator=gen, device="cuda") + 0.5) * K ** -0.5 / 64).half() for _ in w]
+    packed = [EET.preprocess_weights(q) for q in w]
+    x = torch.randn(M, K, generator=gen, device="cuda").half()
+    other = torch.randn(M, N, generator=gen, device="cuda").half()
+
+    stream = torch.cuda.current_stream().cuda_stream
+    gamma = squares = None
+    xn = x
+    if kind.startswith("norm"):
+        # x <- x @ w + x from a small square weight, leaving its sums of squares
+        wx = torch.randint(-127, 128, (K, K), generator=gen, device="cuda", dtype=torch.int8)
+        sx = torch.full((K,), K ** -0.5 / 64, device="cuda").half()
+        h = torch.empty_like(x)
+        squares = torch.full((M, K // 64), float("nan"), device="cuda")
+        check(lib.eet_gemm_w8a16_row(x.data_ptr(), None, None, 0.0, EET.preprocess_weights(wx).data_ptr(), sx.data_ptr(),
+                                     None, None, x.data_ptr(), h.data_ptr(), squares.data_ptr(), M, K, K, stream))
+        assert torch.allclose(squares, h.float().view(M, -1, 64).square().sum(-1), rtol=1e-5)
+        gamma, x = (1 + 0.1 * torch.randn(K, generator=gen, device="cuda")).half(), h
+        xn = torch.empty_like(x)
+        check(lib.eet_rmsnorm(x.data_ptr(), gamma.data_ptr(), xn.data_ptr(), M, K, 1e-6, stream))
+
+    def call():
+        if kind in ("plain", "residual", "gate"):
+            return EET.gemm_w8a16(x, packed[0], s[0], **{"residual": {"residual": other}, "gate": {"gate": other}}.get(kind, {}))
+        out = torch.empty(M, N, dtype=torch.float16, device="cuda")
+        two = kind.endswith("gated")
+        check(lib.eet_gemm_w8a16_row(x.data_ptr(), None if gamma is None else gamma.data_ptr(),
+                                     None if gamma is None else squares.data_ptr(), 1e-6, packed[0].data_ptr(),
+                                     s[0].data_ptr(), packed[1].data_ptr() if two else None, s[1].data_ptr() if two else None,
+                                     None, out.data_ptr(), None, M, N, K, stream))
+        return out
+
+    out = call()
+    y = [(xn.double() @ q.double()) * sc.double() for q, sc in zip(w, s)]
+    # two roundings of each activation, independent: five times their root-mean-square effect on a sum of K products
+    flip = 5 * 2.0 ** -11 * (xn.double() ** 2 @ torch.full((K, 1), 74.0 ** 2, device="cuda").double()).sqrt() * s[0].double().amax() \
+        if gamma is not None else 0.0
+    if kind in ("plain", "residual", "norm"):
+        want = y[0] + (other.double() if kind == "residual" else 0)
+        tol = 2.0 ** -10 * (y[0].abs() + want.abs()) + 1e-4 + flip
+    else:
+        g, u = (y[0], y[1]) if kind.endswith("gated") else (other.double(), y[0])
+        want = torch.nn.functional.silu(g) * u
+        tol = 2.0 ** -10 * (4 * want.abs() + u.abs() + g.abs()) + 1e-4 + flip * (u.abs() + g.abs())
+    assert ((out.double() - want).abs() <= tol).all()
+    assert torch.equal(call(), out)
+    assert _lib.device_status() == 0
+
+
 def test_accumulate_and_fused_finalize_kernels():
     """The decode-path split of the GEMM: sums from eet_gemm_w8a16_accum (two weights in one launch), finished
     by the generic finalize kernel, by the RMSNorm head and by the SwiGLU kernel - each against the oracle."""
