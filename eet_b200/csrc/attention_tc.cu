@@ -108,6 +108,44 @@ __device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint3
     return d;
 }
 
+// The ALiBi bias of one query for 64 keys, requested early: nine aligned 16-byte words that cover the 128 bytes (a row of
+// the bias starts at any even address: its length is the prompt's).  Only words that hold a bias this query needs are
+// read - keys up to min(i, key0 + 63) - so nothing past the tensor is touched; the others count as zero.  40 heads, 2 x 701
+// tokens: 60 us, against 138 with 64 two-byte loads a thread, each touching 32 rows.
+struct PtBias {
+    uint32_t w[36];
+    uint32_t shift;   // bytes from w[0] to the first bias
+
+    __device__ __forceinline__ void load(const __half* row, int key0, int i, bool live)
+    {
+        const uintptr_t first = reinterpret_cast<uintptr_t>(row + key0);
+        const uintptr_t last = reinterpret_cast<uintptr_t>(row + min(i, key0 + kPtK - 1));
+        const uintptr_t base = first & ~(uintptr_t)15;
+        shift = (uint32_t)(first & 15);
+#pragma unroll
+        for (int c = 0; c < 9; ++c) {
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (live && key0 <= i && base + 16 * c <= last) v = __ldg(reinterpret_cast<const uint4*>(base + 16 * c));
+            w[4 * c] = v.x;
+            w[4 * c + 1] = v.y;
+            w[4 * c + 2] = v.z;
+            w[4 * c + 3] = v.w;
+        }
+    }
+    // w[k] becomes the biases of keys key0 + 2 k and key0 + 2 k + 1
+    __device__ __forceinline__ void align()
+    {
+#pragma unroll
+        for (int k = 0; k < 34; ++k) w[k] = (shift & 8) ? w[k + 2] : w[k];
+#pragma unroll
+        for (int k = 0; k < 33; ++k) w[k] = (shift & 4) ? w[k + 1] : w[k];
+        const uint32_t sel = (shift & 2) ? 0x5432u : 0x3210u;
+#pragma unroll
+        for (int k = 0; k < 32; ++k) w[k] = __byte_perm(w[k], w[k + 1], sel);
+    }
+};
+
+template<bool kBias>
 __global__ void __launch_bounds__(kPtThreads, 2)
 prefill_mha_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, __half* __restrict__ ctx, int S, int H,
@@ -243,9 +281,12 @@ prefill_mha_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         const uint32_t t_lane = (uint32_t)lane_base << 16;
         const float scalar = __half2float(__float2half(sqrtf(1.0f / D)));
         float m_run = -1e20f, l_run = 0.f;
+        const __half* arow = kBias ? alibi + ((size_t)h * alibi_stride + (i < S ? i : 0)) * alibi_stride : nullptr;
         bool ok = n_blocks > 0;
         for (int jl = 0; jl < n_blocks && ok; ++jl) {
             const int key0 = (kb_first + jl) * kPtK;
+            PtBias bias;
+            if (kBias) bias.load(arow, key0, i, i < S);   // on its way while the scores are computed
             const uint32_t t_s = tmem + t_lane + kPtColS + (uint32_t)((jl & 1) * kPtK);   // this block's score buffer
             int got = 1;
             if (lane == 0) got = tc_wait(&sm.s_full[jl & 1], (uint32_t)((jl >> 1) & 1), &sm.abort) ? 1 : 0;
@@ -265,25 +306,31 @@ prefill_mha_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             }
 
             float mx = -INFINITY;
-            const __half* arow = (alibi != nullptr && i < S) ? alibi + ((size_t)h * alibi_stride + i) * alibi_stride : nullptr;
             // a block left of the diagonal, right of the padding and inside the prompt needs no per-element mask
-            const bool whole = (key0 + kPtK - 1 <= i) && (key0 >= pad) && (key0 + kPtK <= S) && (arow == nullptr);
+            const bool whole = (key0 + kPtK - 1 <= i) && (key0 >= pad) && (key0 + kPtK <= S);
+            if (kBias) {
+                bias.align();
+#pragma unroll
+                for (int c = 0; c < kPtK; c += 2) {
+                    const float2 b2 = __half22float2(*reinterpret_cast<const __half2*>(&bias.w[c >> 1]));
+                    sc[c] = round_to_half_precision(sc[c] * scalar) + b2.x;
+                    sc[c + 1] = round_to_half_precision(sc[c + 1] * scalar) + b2.y;
+                }
+            }
+            else {
+#pragma unroll
+                for (int c = 0; c < kPtK; ++c) sc[c] = round_to_half_precision(sc[c] * scalar);
+            }
             if (whole) {
 #pragma unroll
-                for (int c = 0; c < kPtK; ++c) {
-                    sc[c] = round_to_half_precision(sc[c] * scalar);
-                    mx = fmaxf(mx, sc[c]);
-                }
+                for (int c = 0; c < kPtK; ++c) mx = fmaxf(mx, sc[c]);
             }
             else {
 #pragma unroll
                 for (int c = 0; c < kPtK; ++c) {
                     const int j = key0 + c;
-                    float v = round_to_half_precision(sc[c] * scalar);
-                    if (arow != nullptr && j <= i) v += __half2float(arow[j]);
-                    v = (j <= i && j >= pad && j < S) ? v : -INFINITY;
-                    sc[c] = v;
-                    mx = fmaxf(mx, v);
+                    sc[c] = (j <= i && j >= pad && j < S) ? sc[c] : -INFINITY;
+                    mx = fmaxf(mx, sc[c]);
                 }
             }
             constexpr float kLog2e = 1.4426950408889634f;
@@ -427,16 +474,17 @@ int launch_prefill_mha_tc(const __half* q, const __half* kcache, const __half* v
     if (int rc = encode_rows_map(&map_q, q, S, (size_t)S, B * H, kPtQ)) return rc;
     if (int rc = encode_rows_map(&map_k, kcache, S, (size_t)T_max, B * H, kPtK)) return rc;
     if (int rc = encode_rows_map(&map_v, vcache, S, (size_t)T_max, B * H, kPtK)) return rc;
-    static bool attr_set[64] = {};
+    auto kern = alibi != nullptr ? prefill_mha_tc_kernel<true> : prefill_mha_tc_kernel<false>;
+    static bool attr_set[64][2] = {};
     int dev = 0;
     EET_CUDA(cudaGetDevice(&dev));
     dev &= 63;
-    if (!attr_set[dev]) {
-        EET_CUDA(cudaFuncSetAttribute(prefill_mha_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPtSmem));
-        attr_set[dev] = true;
+    if (!attr_set[dev][alibi != nullptr]) {
+        EET_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPtSmem));
+        attr_set[dev][alibi != nullptr] = true;
     }
     dim3 grid((S + kPtQ - 1) / kPtQ, B * H);
-    prefill_mha_tc_kernel<<<grid, kPtThreads, kPtSmem, stream>>>(map_q, map_k, map_v, ctx, S, H, pad_len, alibi, alibi_stride);
+    kern<<<grid, kPtThreads, kPtSmem, stream>>>(map_q, map_k, map_v, ctx, S, H, pad_len, alibi, alibi_stride);
     EET_LAUNCH_CHECK();
     return 0;
 }

@@ -177,6 +177,28 @@ def test_prefill_long_prompts(case):
                 assert float(got[b, :, :p_len].abs().max()) == 0.0   # rows inside the padding are zeroed
 
 
+@pytest.mark.parametrize("S,offset", [(96, 0), (97, 1), (129, 3), (191, 6), (255, 7), (320, 2)])
+def test_prefill_bias_at_any_alignment(S, offset):
+    """An arbitrary bias whose rows start at every even address modulo 16 bytes, odd and even row lengths, NaN above the
+    diagonal, and nothing of value around the tensor.  Tolerance as above."""
+    from eet_b200._lib import check, lib
+    B, H, D = 2, 2, 128
+    gen = torch.Generator().manual_seed(S)
+    q, k, v = (torch.randn(B, H, S, D, generator=gen).half() for _ in range(3))
+    bias = (2 * torch.randn(H, S, S, generator=gen)).half()
+    bias[torch.triu(torch.ones(S, S, dtype=torch.bool), 1).expand(H, S, S)] = float("nan")
+    ref = ops.prefill_attention(q, k, v, None, bias)
+    store = torch.full((H * S * S + 16,), float("nan"), dtype=torch.float16, device="cuda")
+    at = store[offset: offset + H * S * S]
+    at.copy_(bias.view(-1))
+    qc, kc, vc = q.cuda(), k.cuda(), v.cuda()
+    ctx = torch.empty(B, S, H * D, dtype=torch.float16, device="cuda")
+    check(lib.eet_prefill_mha(qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), ctx.data_ptr(), B, S, H, D, S, None,
+                              at.data_ptr(), S, _stream()))
+    got = ctx.cpu().view(B, S, H, D).transpose(1, 2)
+    assert torch.allclose(got.float(), ref.float(), atol=4e-3, rtol=4e-3)
+
+
 def test_decode_finishes_projection_sums_itself():
     """qkv given as the fp32 sums of the projection GEMM + per-channel scales: same result as the fp16 form,
     and the sums are zero afterwards."""
