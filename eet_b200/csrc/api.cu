@@ -232,9 +232,10 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
         r.gate = gate;
         return launch_gemm_row(r, (cudaStream_t)stream);
     }
-    // Above 64 tokens a shape that the 256 x 256 kernel can spread over the machine (plain tiles or split-K
-    // clusters) goes there: one launch, epilogue fused, no fp32 scratch.
-    const bool tiles_first = M > 64 && gemm_tc_supported(M, N, K) && tc2_split(M, N, K) > 0;
+    // Above 64 tokens two kernels take most shapes: tiles with the epilogue fused, and stream-K units into the fp32 scratch
+    // with a finishing launch.  The shorter modelled time decides (measured on both sides of the line: 4096 x 11008, M = 256:
+    // tiles 28 us, units 37; 13696 x 5120, M = 256: 52 and 42).
+    const bool tiles_first = M > 64 && gemm_tc_us(M, N, K) < gemm_mid_us(M, N, K);
     if (!tiles_first && M <= mid_use_max_m() && gemm_mid_supported(M, N, K)) {
         // stream-K tensor-core kernel into the fp32 scratch, then one epilogue pass over all rows
         EET_CHECK(ws && aligned16(ws) && ws_bytes >= skinny_sum_bytes(M, N),

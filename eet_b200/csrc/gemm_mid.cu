@@ -429,6 +429,16 @@ bool gemm_mid_supported(int M, int N, int K)
     return M > 16 && M <= kMidMaxM && N % 128 == 0 && K % 64 == 0;
 }
 
+// A fit to measurements at M = 100 ... 512 on the LLaMA-7B and Baichuan-13B shapes (within 8 %): units of 128 channels x 128
+// reduction indices per SM, and 128-token tiles.
+double gemm_mid_us(int M, int N, int K)
+{
+    if (!gemm_mid_supported(M, N, K)) return 1e30;
+    const double units = (double)(N / 128) * ((K / kTile + kMidUnitK - 1) / kMidUnitK) / sm_count();
+    const int t = (M + 127) / 128;
+    return 6.0 + 2.9 * t + (0.38 + 0.38 * t) * units;
+}
+
 // Adds A[M,K] x q(B) (and, with B2, A x q(B2)) into the fp32 buffers a.ws (a.ws2), rows [0, M).
 int launch_gemm_mid(const GemmArgs& a, cudaStream_t stream)
 {

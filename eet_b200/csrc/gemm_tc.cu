@@ -1,27 +1,28 @@
-// W8A16 tensor-core GEMM for the prefill regime (M > 512; smaller M go to the stream-K kernel):
-// C[M,N] = A[M,K] (fp16) x dequant(B), B in the W8T64 layout, per-channel fp16 scale (and optional fp16 residual) in the epilogue.
+// W8A16 tensor-core GEMM for the prefill regime (and from 65 tokens on where its tiles fill the machine better than the
+// stream-K kernel's units): C[M,N] = A[M,K] (fp16) x dequant(B), B in the W8T64 layout, per-channel fp16 scale (and
+// optional fp16 residual or gated activation) in the epilogue.
 //
 // Replaces the reference's fpA_intB GEMM (kernel cutlass_extensions/.../gemm/kernel/fpA_intB_gemm.h:60-486,
 // mainloop .../threadblock/dq_mma_multistage.h:490-583: mma.sync m16n8k16 with int8 -> fp16 conversion in
 // registers after ldmatrix), which has no path for sm_90 or later.
 //
-// B200 design (tcgen05 / TMEM, one CTA per 128-channel x BN-token output tile):
+// B200 design (tcgen05 / TMEM, one CTA per 256-channel x BN-token output tile, BN a multiple of 16 up to 256):
 //  * "swap AB": the weights are the 128-row M operand of tcgen05.mma, the tokens the N operand (BN up to
 //    256), so any batch of tokens fills the tensor core and the per-channel scale is per TMEM lane.
-//  * warp 0 (one lane) is the TMA producer: per 64-wide k-block it requests the two 4 KiB W8T64 tiles of
-//    the 128 channels with 1-D bulk copies and the BN x 64 activation tile with one 2-D tensor-map copy
-//    that lands in the 128-byte-swizzled K-major layout the MMA reads.
-//  * warps 2-5 turn each int8 weight tile into fp16 (prmt + sub.f16x2, exact) and write it into shared
+//  * Per 64-wide k-block the W8T64 tiles of the 256 channels come by 1-D bulk copies and the BN x 64 activation tile by
+//    one 2-D tensor-map copy that lands in the 128-byte-swizzled K-major layout the MMA reads.
+//  * Eight warps turn the int8 weights into fp16 (prmt + sub.f16x2, exact) and write them into shared
 //    memory in the same swizzled K-major layout - the int8 bytes never go through the tensor core as int8
 //    and the weights are never materialised as fp16 in global memory.
-//  * warp 1 (one lane) issues four tcgen05.mma (M128 x BN x K16, fp16 in, fp32 accumulate in TMEM) per
-//    k-block and commits them to the stage's "empty" mbarrier, which releases the stage to the producer.
-//  * after the last k-block warps 2-5 read the accumulator with tcgen05.ld (lane = channel), multiply by
+//  * After the last k-block the same warps read the accumulators with tcgen05.ld (lane = channel), multiply by
 //    the channel's scale, round once to fp16, and pass 128 x 32 blocks through shared memory so that the
 //    stores (and the residual loads) are 16-byte accesses of whole 256-byte row segments.
-//  Three-stage ring of {8 KiB int8 weights, 16 KiB fp16 weights, BN x 128 B activations}.
 //  Every wait is bounded; a wait that runs out sets the device status word, and the CTA still frees its
 //  tensor memory before it returns.
+//
+// Measured and not taken: the fp16 weights in tensor memory as the MMA's A operand (BN up to 192 beside the accumulators,
+// one or two sets of eight conversion warps, two to four buffers): 0.78 us a k-block at BN = 192 and 0.65 at 128, against
+// 0.69 and 0.62 here; moving the bytes alone takes 0.41, i.e. 98 B/ns an SM from L2.
 //
 // Numerics: exact integer weights as fp16, fp32 accumulation, one multiply by the fp16 scale, one rounding
 // to fp16 - the same as the skinny kernel's finalize step.
@@ -35,25 +36,8 @@ namespace eet {
 
 namespace {
 
-constexpr int kTcThreads = 192;     // warp 0 producer, warp 1 MMA issuer + TMEM owner, warps 2-5 transform/epilogue
-constexpr int kTcStages = 3;
 constexpr int kTcW8Bytes = 2 * kTileBytes;          // 128 channels x 64 k, int8
-constexpr int kTcWhBytes = 128 * 128;               // 128 channels x 64 k, fp16, 128 B per row
 constexpr uint32_t kTcSpin = 1u << 24;
-
-__host__ __device__ constexpr int tc_stage_bytes(int bn)
-{
-    return kTcW8Bytes + kTcWhBytes + bn * 128;
-}
-
-struct TcSmem {
-    uint64_t full[kTcStages];    // TMA bytes of a stage have landed (int8 weights + activations)
-    uint64_t ready[kTcStages];   // fp16 weights of a stage are written (4 transform warps)
-    uint64_t empty[kTcStages];   // the MMAs that read a stage have completed (tcgen05.commit)
-    uint64_t accum;              // all MMAs of the tile have completed
-    uint32_t tmem_base;
-    volatile int abort;
-};
 
 // Bounded wait of the warp-specialised kernels.  The roles that issue work are SINGLE threads whose loop
 // is a chain of dependent instructions (a few cycles each at best): the common case - the phase has
@@ -182,164 +166,16 @@ __device__ __forceinline__ void epilogue_block(const uint32_t (&v)[32], float sc
     }
 }
 
-template<int BN>
-__global__ void __launch_bounds__(kTcThreads, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __restrict__ Bw, const __half* __restrict__ scale,
-               __half* __restrict__ C, const __half* __restrict__ residual, int gate, int M, int N, int K)
-{
-    extern __shared__ __align__(1024) uint8_t tc_dyn[];
-    __shared__ TcSmem sm;
-    // the ring must start on a 1024-byte boundary for the swizzled tiles
-    uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_dyn) + 1023) & ~(uintptr_t)1023);
-    constexpr int kStageBytes = tc_stage_bytes(BN);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = blockIdx.x * 128;   // first output channel of the tile
-    const int m0 = blockIdx.y * BN;    // first token of the tile
-    const int KT = K / kTile;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < kTcStages; ++s) {
-            mbar_init(&sm.full[s], 1);
-            mbar_init(&sm.ready[s], 4);
-            mbar_init(&sm.empty[s], 1);
-        }
-        mbar_init(&sm.accum, 1);
-        sm.abort = 0;
-        mbar_fence_init();
-    }
-    if (warp == 1) {
-        // tensor memory: BN fp32 columns x 128 lanes for the accumulator
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)),
-                     "r"((uint32_t)BN)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = sm.tmem_base;
-
-    if (warp == 0) {
-        // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            // (ring positions are counters: this loop is one thread's chain of dependent instructions)
-            int s = 0;
-            uint32_t ph = 1;
-            const uint8_t* w0 = Bw + (size_t)(n0 / kTile) * KT * kTileBytes;
-            for (int kb = 0; kb < KT; ++kb, w0 += kTileBytes) {
-                if (kb >= kTcStages && !tc_wait(&sm.empty[s], ph, &sm.abort)) break;
-                uint8_t* st = ring + (size_t)s * kStageBytes;
-                mbar_arrive_expect_tx(&sm.full[s], (uint32_t)(kTcW8Bytes + BN * 128));
-                bulk_g2s(st, w0, kTileBytes, &sm.full[s]);
-                bulk_g2s(st + kTileBytes, w0 + (size_t)KT * kTileBytes, kTileBytes, &sm.full[s]);
-                tma_load_2d(st + kTcW8Bytes + kTcWhBytes, &tmap_x, kb * kTile, m0, &sm.full[s]);
-                if (++s == kTcStages) {
-                    s = 0;
-                    ph ^= 1;
-                }
-            }
-        }
-    }
-    else if (warp == 1) {
-        // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_f16(128, BN);
-            const uint64_t a_desc0 = umma_desc_sw128(smem_u32(ring + kTcW8Bytes));
-            const uint64_t b_desc0 = umma_desc_sw128(smem_u32(ring + kTcW8Bytes + kTcWhBytes));
-            int s = 0;
-            uint32_t ph = 0;
-            for (int kb = 0; kb < KT; ++kb) {
-                if (!tc_wait(&sm.full[s], ph, &sm.abort)) break;    // activations landed
-                if (!tc_wait(&sm.ready[s], ph, &sm.abort)) break;   // fp16 weights written
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t a_desc = a_desc0 + (uint64_t)(s * (kStageBytes >> 4));
-                const uint64_t b_desc = b_desc0 + (uint64_t)(s * (kStageBytes >> 4));
-                // 16 reduction indices = 32 bytes along the swizzled row: +2 in 16-byte address units
-                umma_f16(tmem, a_desc, b_desc, idesc, kb != 0);
-                umma_f16(tmem, a_desc + 2, b_desc + 2, idesc, true);
-                umma_f16(tmem, a_desc + 4, b_desc + 4, idesc, true);
-                umma_f16(tmem, a_desc + 6, b_desc + 6, idesc, true);
-                umma_commit(&sm.empty[s]);
-                if (++s == kTcStages) {
-                    s = 0;
-                    ph ^= 1;
-                }
-            }
-            umma_commit(&sm.accum);
-        }
-    }
-    else {
-        // ------------------------------------------------------------------ transform warps, then epilogue
-        const int tw = threadIdx.x - 64;          // 0..127
-        int s = 0;
-        uint32_t ph = 0;
-        for (int kb = 0; kb < KT; ++kb) {
-            if (!tc_wait(&sm.full[s], ph, &sm.abort)) break;
-            uint8_t* st = ring + (size_t)s * kStageBytes;
-            const uint8_t* w8 = st;
-            uint8_t* wh = st + kTcW8Bytes;
-#pragma unroll
-            for (int pass = 0; pass < 4; ++pass) {
-                const int r = pass * 32 + (tw >> 2);   // channel row of the tile, 0..127
-                const int qd = tw & 3;                 // 16-byte quarter of its 64 int8 values
-                const uint4 raw = *reinterpret_cast<const uint4*>(w8 + r * 64 + qd * 16);
-                uint4 o0, o1;
-                cvt_u8x4_to_f16x4(raw.x, o0.x, o0.y);
-                cvt_u8x4_to_f16x4(raw.y, o0.z, o0.w);
-                cvt_u8x4_to_f16x4(raw.z, o1.x, o1.y);
-                cvt_u8x4_to_f16x4(raw.w, o1.z, o1.w);
-                uint8_t* row = wh + r * 128;
-                *reinterpret_cast<uint4*>(row + (((2 * qd) ^ (r & 7)) << 4)) = o0;
-                *reinterpret_cast<uint4*>(row + (((2 * qd + 1) ^ (r & 7)) << 4)) = o1;
-            }
-            // make the generic-proxy writes visible to the tensor core (async proxy), then signal
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.ready[s]);
-            if (++s == kTcStages) {
-                s = 0;
-                ph ^= 1;
-            }
-        }
-
-        // ---- epilogue: TMEM lane = channel, columns = tokens ----
-        // every epilogue warp gets here (the waits are bounded); the barrier makes the abort decision uniform
-        tc_wait(&sm.accum, 0, &sm.abort);
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (sm.abort == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int lane_base = (warp & 3) * 32;        // the TMEM lanes this warp may read
-            const float sc = __half2float(scale[n0 + lane_base + lane]);
-            __half* stage = reinterpret_cast<__half*>(ring);
-#pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 32) {
-                if (m0 + c0 >= M) break;
-                uint32_t v[32];
-                tmem_ld32(tmem + ((uint32_t)lane_base << 16) + (uint32_t)c0, v);
-                epilogue_block(v, sc, stage + ((c0 >> 5) & 1) * kEpiStageHalves, lane_base + lane, tw, C, residual,
-                               gate, m0 + c0, M, N, n0);
-            }
-        }
-    }
-
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 1) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)BN) : "memory");
-    }
-}
-
 // ---------------------------------------------------------------------------------------------------
-// Large-M variant: 256 channels x 256 tokens per output tile.  Two accumulators (one per 128-channel half)
-// fill all 512 TMEM columns, and every activation tile fetched from L2 feeds twice as many MMAs as in the
-// kernel above, which halves the L2 -> shared-memory traffic per flop.  The three data streams have their own
-// rings so that each can run as far ahead as its buffer allows:
-//   activations : 3 x 32 KiB, one 2-D TMA copy per k-block            (warp 0)
-//   int8 weights: 4 x 16 KiB, four 4 KiB bulk copies per k-block      (warp 6)
+// Two accumulators (one per 128-channel half) fill the TMEM columns, and every activation tile fetched from L2 feeds both
+// halves.  The three data streams have their own rings so that each can run as far ahead as its buffer allows (the launcher
+// deals what shared memory has: BN = 256 three stages of activations and four of weights, BN = 128 five of each):
+//   activations : BN x 128 bytes a stage, one 2-D TMA copy per k-block            (warp 0)
+//   int8 weights: 16 KiB, four 4 KiB bulk copies per k-block                     (warp 6)
 //   fp16 weights: 2 x 32 KiB (k-block x two 128-channel halves), written by warps 2-5 / 7-10, read by tcgen05.mma
-// One commit per k-block ("done", ring of 6 = lcm of the ring depths) releases the activation stage to its
+// One commit per k-block ("done") releases the activation stage to its
 // producer and the fp16 stage to the transform warps: the issuing thread pays for two waits, eight MMAs and
-// one commit per k-block.
+// one commit per k-block.  N is a multiple of 128: the last tile of a row may have a lower half only.
 //
 // Two ways to spread the tiles over the SMs:
 //
@@ -356,7 +192,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __rest
 //     read the same tiles at the same time (4096^2, M = 4096: 145 us against 109); (ii) whole tiles in waves and
 //     only the left-over tiles cut along K into pieces that keep the k-blocks in step gained 0-3 % (4096 x 12288,
 //     M = 4096: 328 us against 330; 11008 x 4096: 267 against 274) - exporting and importing 256 KiB accumulators
-//     costs what the shorter wave saves.
+//     costs what the shorter wave saves.  What helps is a BN whose waves come out even (tc2_plan): 13696 x 5120 at M = 999
+//     is 140 tiles of 144 tokens in one wave, 144 us, where 80 tiles of 256 found no form at all (264 us in a kernel
+//     of 128-channel tiles that is gone).
 //
 // (b) Split-K over a thread-block cluster (gridDim.z = cluster size S = 2, 3 or 4) for shapes with fewer tiles
 //     than SMs: the S CTAs of a cluster share one output tile (tile0 + blockIdx.x) and each walks 1/S of the
@@ -367,9 +205,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __rest
 //     the S - 1 partials to its own accumulator in rank order and runs the usual epilogue for its blocks only.
 // ---------------------------------------------------------------------------------------------------
 constexpr int kTc2Threads = 352;   // X producer, MMA issuer, 4 + 4 transform/epilogue warps, W producer
-constexpr int kTc2NX = 3, kTc2NW = 4, kTc2NH = 2, kTc2ND = 6;
-constexpr int kTc2XBytes = 256 * 128, kTc2WBytes = 4 * kTileBytes, kTc2HBytes = 128 * 128;   // H: one half
-constexpr int kTc2Smem = kTc2NX * kTc2XBytes + kTc2NW * kTc2WBytes + kTc2NH * 2 * kTc2HBytes;
+constexpr int kTc2MaxNX = 8, kTc2MaxNW = 8, kTc2NH = 2, kTc2ND = 8;
+constexpr int kTc2WBytes = 4 * kTileBytes, kTc2HBytes = 128 * 128;   // H: one half
+constexpr int kTc2Smem = 224 * 1024;
 constexpr int kTc2RedBlock = 256 * 128;               // one partial block: 256 channels x 32 tokens fp32
 constexpr int kTc2StageBytes = 2 * 2 * kEpiStageHalves * 2;   // the epilogue's fp16 staging tiles (two per group)
 // cluster mode: partial blocks received by one CTA (blocks owned, at most ceil(8 / S), x (S - 1) senders) follow
@@ -396,8 +234,8 @@ __device__ __forceinline__ bool epi_bar_or(bool pred)
 }
 
 struct Tc2Smem {
-    uint64_t x_full[kTc2NX];
-    uint64_t w_full[kTc2NW], w_empty[kTc2NW];
+    uint64_t x_full[kTc2MaxNX];
+    uint64_t w_full[kTc2MaxNW], w_empty[kTc2MaxNW];
     uint64_t h_ready[kTc2NH];     // both halves of a k-block are written (8 transform warps)
     uint64_t done[kTc2ND];        // the MMAs of a k-block have completed
     uint64_t accum;               // all MMAs of a segment have completed
@@ -435,8 +273,8 @@ struct Tc2Work {
 
 __global__ void __launch_bounds__(kTc2Threads, 1)
 gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __restrict__ Bw, const __half* __restrict__ scale,
-                __half* __restrict__ C, const __half* __restrict__ residual, int gate, int M, int N, int K, int tile0,
-                int tile_count)
+                __half* __restrict__ C, const __half* __restrict__ residual, int gate, int M, int N, int K, int bn, int nx, int nw,
+                int tile0, int tile_count)
 {
     // This launch covers tiles [tile0, tile0 + tile_count) of the output, numbered row-major over (token tile,
     // channel tile).
@@ -444,11 +282,12 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
     __shared__ Tc2Smem sm;
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_dyn) + 1023) & ~(uintptr_t)1023);
     uint8_t* x_ring = base;                                   // 1024-byte aligned tiles (swizzled)
-    uint8_t* h_ring = base + kTc2NX * kTc2XBytes;             // 1024-byte aligned tiles (swizzled)
+    const int x_bytes = bn * 128;                             // one k-block of activations
+    uint8_t* h_ring = base + (size_t)nx * x_bytes;            // 1024-byte aligned tiles (swizzled)
     uint8_t* w_ring = h_ring + kTc2NH * 2 * kTc2HBytes;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int S = (int)gridDim.z, rank = (int)blockIdx.z;
-    const int tiles_n = N / 256, tiles_m = (M + 255) / 256;
+    const int tiles_n = (N + 255) / 256;
 
     Tc2Work wk;
     wk.KT = K / kTile;
@@ -467,14 +306,13 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
     else {
         wk.nseg = (tile_count - wk.i + wk.G - 1) / wk.G;   // tiles tile0 + i, tile0 + i + G, ...
     }
-    (void)tiles_m;
     const int nseg = wk.nseg;
 
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kTc2NX; ++s) mbar_init(&sm.x_full[s], 1);
+        for (int s = 0; s < nx; ++s) mbar_init(&sm.x_full[s], 1);
         for (int s = 0; s < kTc2ND; ++s) mbar_init(&sm.done[s], 1);
-        for (int s = 0; s < kTc2NW; ++s) {
+        for (int s = 0; s < nw; ++s) {
             mbar_init(&sm.w_full[s], 1);
             mbar_init(&sm.w_empty[s], 8);
         }
@@ -506,9 +344,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
             pdl_wait();            // the activations are the preceding kernel's output (the weights are not)
             for (int p = 0; p < nseg && ok; ++p) {
                 const Tc2Seg sg = wk.seg(p);
-                const int m0 = (sg.tile / tiles_n) * 256;
+                const int m0 = (sg.tile / tiles_n) * bn;
                 for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
-                    if (it >= kTc2NX) {
+                    if (it >= nx) {
                         if (!tc_wait(&sm.done[d], phd, &sm.abort)) {
                             ok = false;
                             break;
@@ -518,9 +356,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
                             phd ^= 1;
                         }
                     }
-                    mbar_arrive_expect_tx(&sm.x_full[s], (uint32_t)kTc2XBytes);
-                    tma_load_2d(x_ring + (size_t)s * kTc2XBytes, &tmap_x, kb * kTile, m0, &sm.x_full[s]);
-                    if (++s == kTc2NX) s = 0;
+                    mbar_arrive_expect_tx(&sm.x_full[s], (uint32_t)x_bytes);
+                    tma_load_2d(x_ring + (size_t)s * x_bytes, &tmap_x, kb * kTile, m0, &sm.x_full[s]);
+                    if (++s == nx) s = 0;
                 }
             }
         }
@@ -534,19 +372,20 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
             for (int p = 0; p < nseg && ok; ++p) {
                 const Tc2Seg sg = wk.seg(p);
                 const int n0 = (sg.tile % tiles_n) * 256;
+                const int rows = n0 + 128 < N ? 4 : 2;   // tile rows of 64 channels
                 const uint8_t* w0 = Bw + ((size_t)(n0 / kTile) * wk.KT + sg.kb0) * kTileBytes;
                 for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it, w0 += kTileBytes) {
-                    if (it >= kTc2NW && !tc_wait(&sm.w_empty[s], ph, &sm.abort)) {
+                    if (it >= nw && !tc_wait(&sm.w_empty[s], ph, &sm.abort)) {
                         ok = false;
                         break;
                     }
-                    mbar_arrive_expect_tx(&sm.w_full[s], (uint32_t)kTc2WBytes);
+                    mbar_arrive_expect_tx(&sm.w_full[s], (uint32_t)(rows * kTileBytes));
                     uint8_t* dst = w_ring + (size_t)s * kTc2WBytes;
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        bulk_g2s(dst + i * kTileBytes, w0 + (size_t)i * wk.KT * kTileBytes, kTileBytes, &sm.w_full[s]);
+                        if (i < rows) bulk_g2s(dst + i * kTileBytes, w0 + (size_t)i * wk.KT * kTileBytes, kTileBytes, &sm.w_full[s]);
                     }
-                    if (++s == kTc2NW) {
+                    if (++s == nw) {
                         s = 0;
                         ph ^= 1;
                     }
@@ -557,7 +396,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
     else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
         if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_f16(128, 256);
+            const uint32_t idesc = umma_idesc_f16(128, bn);
             const uint64_t b_desc0 = umma_desc_sw128(smem_u32(x_ring));
             const uint64_t a_desc0 = umma_desc_sw128(smem_u32(h_ring));
             int sx = 0, sd = 0, it = 0;
@@ -565,6 +404,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
             bool ok = true;
             for (int p = 0; p < nseg && ok; ++p) {
                 const Tc2Seg sg = wk.seg(p);
+                const bool upper = (sg.tile % tiles_n) * 256 + 128 < N;
                 // the accumulators are overwritten: the epilogue of the previous segment must have read them
                 if (p > 0 && !tc_wait(&sm.acc_free, (uint32_t)((p - 1) & 1), &sm.abort)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -576,7 +416,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t b_desc = b_desc0 + (uint64_t)(sx * (kTc2XBytes >> 4));
+                    const uint64_t b_desc = b_desc0 + (uint64_t)(sx * (x_bytes >> 4));
                     const uint64_t a0 = a_desc0 + (uint64_t)(sh * (2 * kTc2HBytes >> 4));
                     const uint64_t a1 = a0 + (uint64_t)(kTc2HBytes >> 4);
                     const bool acc = kb != sg.kb0;
@@ -584,13 +424,15 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
                     umma_f16(tmem, a0 + 2, b_desc + 2, idesc, true);
                     umma_f16(tmem, a0 + 4, b_desc + 4, idesc, true);
                     umma_f16(tmem, a0 + 6, b_desc + 6, idesc, true);
-                    umma_f16(tmem + 256, a1, b_desc, idesc, acc);
-                    umma_f16(tmem + 256, a1 + 2, b_desc + 2, idesc, true);
-                    umma_f16(tmem + 256, a1 + 4, b_desc + 4, idesc, true);
-                    umma_f16(tmem + 256, a1 + 6, b_desc + 6, idesc, true);
+                    if (upper) {
+                        umma_f16(tmem + 256, a1, b_desc, idesc, acc);
+                        umma_f16(tmem + 256, a1 + 2, b_desc + 2, idesc, true);
+                        umma_f16(tmem + 256, a1 + 4, b_desc + 4, idesc, true);
+                        umma_f16(tmem + 256, a1 + 6, b_desc + 6, idesc, true);
+                    }
                     umma_commit(&sm.done[sd]);
                     if (++sd == kTc2ND) sd = 0;
-                    if (++sx == kTc2NX) {
+                    if (++sx == nx) {
                         sx = 0;
                         phx ^= 1;
                     }
@@ -613,6 +455,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
         bool ok = true;
         for (int p = 0; p < nseg && ok; ++p) {
             const Tc2Seg sg = wk.seg(p);
+            const bool mine = grp == 0 || (sg.tile % tiles_n) * 256 + 128 < N;   // (the last tile may have no upper half)
             for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
                 if (!tc_wait(&sm.w_full[sw], phw, &sm.abort)) {
                     ok = false;
@@ -620,6 +463,23 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
                 }
                 const uint8_t* w8 = w_ring + (size_t)sw * kTc2WBytes;
                 const int sh = it & 1;
+                // (converted before the wait for the buffer: what follows that wait is on the chain from one k-block's
+                // MMAs to the next but one's)
+                uint4 o[4][2];
+                const int qd = tw & 3;
+                if (mine) {
+#pragma unroll
+                    for (int pass = 0; pass < 4; ++pass) {
+                        const int r = pass * 32 + (tw >> 2);   // channel row of this half, 0..127
+                        const uint4 raw = *reinterpret_cast<const uint4*>(w8 + (grp * 128 + r) * 64 + qd * 16);
+                        cvt_u8x4_to_f16x4(raw.x, o[pass][0].x, o[pass][0].y);
+                        cvt_u8x4_to_f16x4(raw.y, o[pass][0].z, o[pass][0].w);
+                        cvt_u8x4_to_f16x4(raw.z, o[pass][1].x, o[pass][1].y);
+                        cvt_u8x4_to_f16x4(raw.w, o[pass][1].z, o[pass][1].w);
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm.w_empty[sw]);
                 if (it >= kTc2NH) {
                     if (!tc_wait(&sm.done[d], phd, &sm.abort)) {
                         ok = false;
@@ -630,28 +490,22 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
                         phd ^= 1;
                     }
                 }
-                uint8_t* wh = h_ring + (size_t)(sh * 2 + grp) * kTc2HBytes;
+                if (mine) {
+                    uint8_t* wh = h_ring + (size_t)(sh * 2 + grp) * kTc2HBytes;
 #pragma unroll
-                for (int pass = 0; pass < 4; ++pass) {
-                    const int r = pass * 32 + (tw >> 2);   // channel row of this half, 0..127
-                    const int qd = tw & 3;
-                    const uint4 raw = *reinterpret_cast<const uint4*>(w8 + (grp * 128 + r) * 64 + qd * 16);
-                    uint4 o0, o1;
-                    cvt_u8x4_to_f16x4(raw.x, o0.x, o0.y);
-                    cvt_u8x4_to_f16x4(raw.y, o0.z, o0.w);
-                    cvt_u8x4_to_f16x4(raw.z, o1.x, o1.y);
-                    cvt_u8x4_to_f16x4(raw.w, o1.z, o1.w);
-                    uint8_t* row = wh + r * 128;
-                    *reinterpret_cast<uint4*>(row + (((2 * qd) ^ (r & 7)) << 4)) = o0;
-                    *reinterpret_cast<uint4*>(row + (((2 * qd + 1) ^ (r & 7)) << 4)) = o1;
+                    for (int pass = 0; pass < 4; ++pass) {
+                        const int r = pass * 32 + (tw >> 2);
+                        uint8_t* row = wh + r * 128;
+                        *reinterpret_cast<uint4*>(row + (((2 * qd) ^ (r & 7)) << 4)) = o[pass][0];
+                        *reinterpret_cast<uint4*>(row + (((2 * qd + 1) ^ (r & 7)) << 4)) = o[pass][1];
+                    }
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) {
                     mbar_arrive(&sm.h_ready[sh]);
-                    mbar_arrive(&sm.w_empty[sw]);
                 }
-                if (++sw == kTc2NW) {
+                if (++sw == nw) {
                     sw = 0;
                     phw ^= 1;
                 }
@@ -671,24 +525,23 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             pdl_wait();   // the output and the residual belong to the dependency chain
-            const int n0 = (sg.tile % tiles_n) * 256, m0 = (sg.tile / tiles_n) * 256;
-            {
+            const int n0 = (sg.tile % tiles_n) * 256, m0 = (sg.tile / tiles_n) * bn;
+            const int m1 = min(M, m0 + bn);
+            if (mine) {
                 const float sc = __half2float(scale[n0 + ch]);
                 __half* stage = reinterpret_cast<__half*>(h_ring) + grp * 2 * kEpiStageHalves;
                 int blk = 0;
 #pragma unroll 1
-                for (int b = 0; b < 8; ++b, ++blk) {
-                    const int c0 = 32 * b;
-                    if (m0 + c0 >= M) break;
+                for (int c0 = 0; m0 + c0 < m1; c0 += 32, ++blk) {
                     uint32_t v[32];
                     tmem_ld32(tmem + ((uint32_t)lane_base << 16) + (uint32_t)(grp * 256 + c0), v);
                     if (grp == 0) {
                         epilogue_block<1>(v, sc, stage + (blk & 1) * kEpiStageHalves, lane_base + lane, tw, C, residual, gate,
-                                          m0 + c0, M, N, n0);
+                                          m0 + c0, m1, N, n0);
                     }
                     else {
                         epilogue_block<2>(v, sc, stage + (blk & 1) * kEpiStageHalves, lane_base + lane, tw, C, residual, gate,
-                                          m0 + c0, M, N, n0 + 128);
+                                          m0 + c0, m1, N, n0 + 128);
                     }
                 }
                 // The staging tiles lie in this group's own part of the fp16 weight ring: its next conversions
@@ -715,14 +568,15 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
         const int tw = (warp - (grp ? 7 : 2)) * 32 + lane;   // 0..127 within the group
         const int lane_base = (warp & 3) * 32;
         const int ch = grp * 128 + lane_base + lane;          // this thread's channel of the tile
-        const int n0 = (wk.cluster_tile % tiles_n) * 256, m0 = (wk.cluster_tile / tiles_n) * 256;
+        const int n0 = (wk.cluster_tile % tiles_n) * 256, m0 = (wk.cluster_tile / tiles_n) * bn;
+        const int m1 = min(M, m0 + bn);
+        if (grp == 1 && n0 + 128 >= N) epi_live = false;      // the last tile may have no upper half
         uint8_t* red = base + kTc2StageBytes;
         // All CTAs of the cluster have completed their MMAs: their rings may be overwritten.
         cooperative_groups::this_cluster().sync();
         if (epi_warp && epi_live) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int b = 0; b < 8; ++b) {
-                if (m0 + 32 * b >= M) break;
+            for (int b = 0; m0 + 32 * b < m1; ++b) {
                 const int owner = b % S;
                 if (owner == rank) continue;
                 uint32_t v[32];
@@ -749,9 +603,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
             const float sc = __half2float(scale[n0 + ch]);
             int blk = 0;
 #pragma unroll 1
-            for (int b = rank; b < 8; b += S, ++blk) {
+            for (int b = rank; m0 + 32 * b < m1; b += S, ++blk) {
                 const int c0 = 32 * b;
-                if (m0 + c0 >= M) break;
                 uint32_t v[32];
                 tmem_ld32(tmem + ((uint32_t)lane_base << 16) + (uint32_t)(grp * 256 + c0), v);
                 for (int src = 0; src < S - 1; ++src) {
@@ -766,11 +619,11 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
                     }
                 }
                 if (grp == 0) {
-                    epilogue_block<1>(v, sc, stage + (blk & 1) * kEpiStageHalves, lane_base + lane, tw, C, residual, gate, m0 + c0, M,
+                    epilogue_block<1>(v, sc, stage + (blk & 1) * kEpiStageHalves, lane_base + lane, tw, C, residual, gate, m0 + c0, m1,
                                       N, n0);
                 }
                 else {
-                    epilogue_block<2>(v, sc, stage + (blk & 1) * kEpiStageHalves, lane_base + lane, tw, C, residual, gate, m0 + c0, M,
+                    epilogue_block<2>(v, sc, stage + (blk & 1) * kEpiStageHalves, lane_base + lane, tw, C, residual, gate, m0 + c0, m1,
                                       N, n0 + 128);
                 }
             }
@@ -802,33 +655,12 @@ EncodeTiledFn encode_tiled_fn()
     return fn;
 }
 
-template<int BN>
-int launch_tc(const CUtensorMap& map, const uint8_t* B, const __half* scale, __half* C, const __half* residual, int gate,
-              int M, int N, int K, cudaStream_t stream)
-{
-    static bool attr_set[64] = {};
-    int dev = 0;
-    EET_CUDA(cudaGetDevice(&dev));
-    dev &= 63;
-    const size_t smem = (size_t)kTcStages * tc_stage_bytes(BN) + 1024;
-    if (!attr_set[dev]) {
-        EET_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set[dev] = true;
-    }
-    dim3 grid(N / 128, (M + BN - 1) / BN);
-    gemm_tc_kernel<BN><<<grid, kTcThreads, smem, stream>>>(map, B, scale, C, residual, gate, M, N, K);
-    EET_LAUNCH_CHECK();
-    return 0;
-}
-
 }  // namespace
 
-// Smallest M these kernels accept.  The dispatcher sends M <= 512 to the stream-K kernel first; only shapes
-// that kernel does not take can arrive here with fewer tokens, and below 65 a one-tile-per-CTA kernel would
-// leave most SMs idle, so the skinny kernel serves those.
+// Smallest M this kernel accepts: below, the stream-K and skinny kernels serve.
 constexpr int kTcMinM = 65;
 
-// Clusters of `split` CTAs of the 256 x 256 kernel that can be resident at once (0: that cluster size cannot be
+// Clusters of `split` CTAs of the kernel that can be resident at once (0: that cluster size cannot be
 // launched), asked of the occupancy calculator once per device and size.
 static int tc2_max_clusters(int split)
 {
@@ -861,43 +693,63 @@ static int tc2_max_clusters(int split)
     return cached[dev][split] > 0 ? cached[dev][split] : 0;
 }
 
-// Largest cluster size (4, 3, 2) over which the k-blocks of each of `tiles` tiles can be split: all clusters
-// resident at once, at least four k-blocks per CTA; 0 if none.  (Clusters of 8 were measured too: the all-to-all
-// of 7/8 of every accumulator costs more than the shorter k-loops save.)
-static int tc2_cluster_size(int tiles, int K)
+// How a shape is run: BN tokens per tile; the first `whole` tiles on persistent CTAs, the others (none, the last partial
+// wave, or all) with their k-blocks split over clusters of `split` CTAs; and the modelled time in microseconds.
+struct Tc2Plan {
+    int bn, tiles, whole, split;
+    double us;
+};
+
+// Time of a k-block of a 256 x BN tile with the machine full, measured at BN = 64 ... 256 on 4096 x 12288.  Below 128 tokens
+// the conversion of the weights and the hand-overs set the pace, above it the tensor core and shared memory.
+static double tc2_block_us(int bn)
 {
-    const int KT = K / kTile;
-    static const int sizes[3] = {4, 3, 2};
-    for (int i = 0; i < 3; ++i) {
-        const int sp = sizes[i];
-        if (KT / sp >= 4 && tiles <= tc2_max_clusters(sp)) return sp;
-    }
-    return 0;
+    static const double at[9] = {0.57, 0.57, 0.58, 0.60, 0.62, 0.647, 0.69, 0.753, 0.80};   // at 0, 32, ..., 256
+    const int i = bn / 32;
+    return at[i] + (i < 8 ? (at[i + 1] - at[i]) * (bn % 32) / 32.0 : 0.0);
 }
 
-// How the 256 x 256 kernel would run this shape: 0 = not at all, 1 = whole tiles on persistent CTAs, 2/3/4 = the
-// k-blocks of a tile split over a cluster of that size.  Whole tiles need most of the machine's worth of them
-// (120); below that the largest split is taken that puts at least 96 CTAs to work, whose clusters are all
-// resident at once and which still leaves each CTA four k-blocks.
-int tc2_split(int M, int N, int K)
+// The plan with the least modelled time over all BN and ways to treat the tiles that fill no wave.  A launch costs 5.5 us
+// around its tiles, a tile's epilogue is not overlapped with its CTA's next tile, a cluster pays for two barriers and the
+// exchange of partial sums, a second launch for its start.  Against measurements at M = 100 ... 4096 on the LLaMA-7B and
+// Baichuan-13B shapes the model is within 10 %.
+static Tc2Plan tc2_plan(int M, int N, int K)
 {
-    if (N % 256 != 0 || M < kTcMinM) return 0;
+    const int KT = K / kTile, G = sm_count();
+    const int tiles_n = (N + 255) / 256;
     static int forced = -2;
     if (forced == -2) {
         const char* e = getenv("EET_TC2_SPLIT");
         forced = e ? atoi(e) : -1;
     }
-    const long long tiles = (long long)(N / 256) * ((M + 255) / 256);
-    if (forced == 0) return tiles >= 120 ? 1 : 0;
-    if (tiles >= 120) return 1;
-    const int sp = tc2_cluster_size((int)tiles, K);
-    if (forced > 0) return (sp > 0 && K / kTile / forced >= 4 && tiles <= tc2_max_clusters(forced)) ? forced : 0;
-    return (sp > 1 && tiles * sp >= 96) ? sp : 0;
+    Tc2Plan best = {0, 0, 0, 1, 1e30};
+    for (int bn = M < 256 ? (M + 15) / 16 * 16 : 256; bn >= 32; bn -= 16) {
+        const long long tiles_ll = (long long)tiles_n * ((M + bn - 1) / bn);
+        if (tiles_ll > 0x7fffffffLL) continue;
+        const int tiles = (int)tiles_ll;
+        const double block = tc2_block_us(bn), epilogue = 1.5 + 0.01 * bn;
+        for (int sp = 1; sp <= 4; ++sp) {
+            const int left = sp > 1 ? tiles % G : 0, whole = tiles - left;
+            if (sp > 1 && (left == 0 || KT / sp < 4 || left > tc2_max_clusters(sp))) continue;
+            if (forced >= 0 && sp != 1 && sp != forced) continue;
+            double us = 5.5 + (double)((whole + G - 1) / G) * (KT * block + epilogue);
+            if (left > 0) us += (KT + sp - 1) / sp * block + epilogue + 4.0 + (whole > 0 ? 2.0 : 0.0);
+            if (forced == sp && sp > 1 && whole == 0) us *= 0.1;
+            if (us < best.us) best = Tc2Plan{bn, tiles, whole, sp, us};
+        }
+    }
+    return best;
 }
 
 bool gemm_tc_supported(int M, int N, int K)
 {
     return M >= kTcMinM && N % 128 == 0 && K % 64 == 0;
+}
+
+// Modelled time in microseconds; a large number where the kernel does not take the shape.
+double gemm_tc_us(int M, int N, int K)
+{
+    return gemm_tc_supported(M, N, K) ? tc2_plan(M, N, K).us : 1e30;
 }
 
 int launch_gemm_tc(const __half* A, const uint8_t* B, const __half* scale, __half* C, const __half* residual, int gate,
@@ -906,70 +758,56 @@ int launch_gemm_tc(const __half* A, const uint8_t* B, const __half* scale, __hal
     EET_CHECK(gemm_tc_supported(M, N, K), "tensor-core GEMM: needs M >= 65, N %% 128 == 0, K %% 64 == 0");
     EncodeTiledFn encode = encode_tiled_fn();
     EET_CHECK(encode != nullptr, "tensor-core GEMM: cuTensorMapEncodeTiled is not available from the driver");
-    const int split = tc2_split(M, N, K);
-    // token rows per activation tile: always 256 for the 256 x 256 kernel (rows past M read as zeros)
-    const int bn = (split > 0 || M > 128) ? 256 : (M > 64 ? 128 : 64);
+    static bool attr_set[64] = {};
+    int dev = 0;
+    EET_CUDA(cudaGetDevice(&dev));
+    dev &= 63;
+    const size_t smem = (size_t)kTc2Smem + 1024;
+    if (!attr_set[dev]) {
+        EET_CUDA(cudaFuncSetAttribute(gemm_tc2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        attr_set[dev] = true;
+    }
+    const Tc2Plan plan = tc2_plan(M, N, K);
+    EET_CHECK(plan.bn > 0, "tensor-core GEMM: no plan for M=%d N=%d K=%d", M, N, K);
     CUtensorMap map;
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
     const cuuint64_t strides[1] = {(cuuint64_t)K * sizeof(__half)};
-    const cuuint32_t box[2] = {64, (cuuint32_t)bn};
+    const cuuint32_t box[2] = {64, (cuuint32_t)plan.bn};   // (rows past M read as zeros)
     const cuuint32_t elem[2] = {1, 1};
     const CUresult rc = encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(A), dims, strides, box, elem,
                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     EET_CHECK(rc == CUDA_SUCCESS, "tensor-core GEMM: cuTensorMapEncodeTiled failed with code %d", (int)rc);
-    // the 256 x 256 tiles pay off once there are enough of them to fill most of the machine - on a grid of
-    // persistent CTAs, or with the k-blocks of a tile split over a cluster
-    if (split > 0) {
-        static bool attr_set2[64] = {};
-        int dev = 0;
-        EET_CUDA(cudaGetDevice(&dev));
-        dev &= 63;
-        const size_t smem = (size_t)kTc2Smem + 1024;
-        if (!attr_set2[dev]) {
-            EET_CUDA(cudaFuncSetAttribute(gemm_tc2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            attr_set2[dev] = true;
-        }
-        const int tiles = (N / 256) * ((M + 255) / 256);
-        auto launch = [&](int tile0, int count, int grid_x, int cluster) -> cudaError_t {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)grid_x, 1, (unsigned)cluster);
-            cfg.blockDim = dim3(kTc2Threads, 1, 1);
-            cfg.dynamicSmemBytes = smem;
-            cfg.stream = stream;
-            cudaLaunchAttribute attr[2];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = 1;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = (unsigned)cluster;
-            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[1].val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 2;
-            return cudaLaunchKernelEx(&cfg, gemm_tc2_kernel, map, B, scale, C, residual, gate, M, N, K, tile0, count);
-        };
-        if (split > 1) {
-            EET_CUDA(launch(0, tiles, tiles, split));
-            return 0;
-        }
-        // Whole tiles on one persistent CTA per SM (fewer when there are fewer tiles).  When the last wave would
-        // be at most half full, its tiles go to a second launch that splits each over a cluster instead: a
-        // quarter or a third of the k-blocks per CTA rather than a full tile's worth on a fifth of the SMs.
-        const int G = tiles < sm_count() ? tiles : sm_count();
-        const int left = tiles % G;
-        const int left_split = (left > 0 && 2 * left <= G) ? tc2_cluster_size(left, K) : 0;
-        if (left_split > 1) {
-            EET_CUDA(launch(0, tiles - left, G, 1));
-            EET_CUDA(launch(tiles - left, left, left, left_split));
-        }
-        else {
-            EET_CUDA(launch(0, tiles, G, 1));
-        }
-        return 0;
+    // the rings share what the fp16 weights (64 KiB) leave: as many stages of both as fit, the rest to the int8 weights
+    const int x_bytes = plan.bn * 128, room = kTc2Smem - kTc2NH * 2 * kTc2HBytes;
+    int nx = room / (x_bytes + kTc2WBytes);
+    if (nx > kTc2MaxNX) nx = kTc2MaxNX;
+    int nw = (room - nx * x_bytes) / kTc2WBytes;
+    if (nw > kTc2MaxNW) nw = kTc2MaxNW;
+    auto launch = [&](int tile0, int count, int grid_x, int cluster) -> cudaError_t {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)grid_x, 1, (unsigned)cluster);
+        cfg.blockDim = dim3(kTc2Threads, 1, 1);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = (unsigned)cluster;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        return cudaLaunchKernelEx(&cfg, gemm_tc2_kernel, map, B, scale, C, residual, gate, M, N, K, plan.bn, nx, nw, tile0, count);
+    };
+    if (plan.whole > 0) {
+        EET_CUDA(launch(0, plan.whole, plan.whole < sm_count() ? plan.whole : sm_count(), 1));
     }
-    if (bn == 256) return launch_tc<256>(map, B, scale, C, residual, gate, M, N, K, stream);
-    if (bn == 128) return launch_tc<128>(map, B, scale, C, residual, gate, M, N, K, stream);
-    return launch_tc<64>(map, B, scale, C, residual, gate, M, N, K, stream);
+    if (plan.whole < plan.tiles) {
+        EET_CUDA(launch(plan.whole, plan.tiles - plan.whole, plan.tiles - plan.whole, plan.split));
+    }
+    return 0;
 }
 
 }  // namespace eet

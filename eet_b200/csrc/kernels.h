@@ -50,7 +50,7 @@ int launch_gemm_row(RowGemmArgs a, cudaStream_t stream);
 
 // gemm_tc.cu (tcgen05 / TMEM)
 bool gemm_tc_supported(int M, int N, int K);
-int tc2_split(int M, int N, int K);  // 0: the 256 x 256 kernel does not take this shape; else its split-K cluster size
+double gemm_tc_us(int M, int N, int K);  // modelled time in microseconds (large: the kernel does not take the shape)
 int launch_gemm_tc(const __half* A, const uint8_t* B, const __half* scale, __half* C, const __half* residual, int gate,
                    int M, int N, int K, cudaStream_t stream);
 
@@ -58,6 +58,7 @@ int launch_gemm_tc(const __half* A, const uint8_t* B, const __half* scale, __hal
 constexpr int kMidMaxM = 512;
 bool gemm_mid_supported(int M, int N, int K);
 int launch_gemm_mid(const GemmArgs& a, cudaStream_t stream);
+double gemm_mid_us(int M, int N, int K);  // modelled time with the finishing launch (large: the kernel does not take the shape)
 
 // noalloc.cu
 int gemm_w8a16_noalloc(const __half* A, const uint8_t* B, const __half* scale, __half* C, int M, int N, int K,

@@ -110,6 +110,34 @@ def test_empty_and_invalid():
     assert rc != 0
 
 
+@pytest.mark.parametrize("kind", ["plain", "residual", "gate"])
+@pytest.mark.parametrize("K,N,M", [(64, 128, 65), (320, 384, 97), (1024, 640, 513), (4096, 4224, 130), (640, 13696, 999),
+                                   (2048, 896, 4095), (5120, 256, 700), (13696, 5120, 600), (192, 38016, 259)])
+def test_prefill_gemm_tiles(K, N, M, kind):
+    """Tiles with a lower half only, token tiles that are no multiple of 32, whole waves, waves with a split remainder and
+    split tiles only, few k-blocks.  Bound: fp32 sums, one fp16 rounding of the product and one of the sum with the
+    residual, 2^-11 each, doubled; the activation's error is its operands' plus its own three fp16 steps."""
+    from eet_b200 import EET, _lib
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    q = torch.randint(-127, 128, (K, N), generator=gen, device="cuda", dtype=torch.int8)
+    s = ((torch.rand(N, generator=gen, device="cuda") + 0.5) * K ** -0.5 / 64).half()
+    x = torch.randn(M, K, generator=gen, device="cuda").half()
+    other = torch.randn(M, N, generator=gen, device="cuda").half()
+    out = torch.full((M + 1, N), 7.0, dtype=torch.float16, device="cuda")
+    kw = {"residual": {"residual": other}, "gate": {"gate": other}}.get(kind, {})
+    EET.gemm_w8a16(x, EET.preprocess_weights(q), s, out=out[:M], **kw)
+    y = (x.double() @ q.double()) * s.double()
+    if kind == "gate":
+        want = torch.nn.functional.silu(other.double()) * y
+        tol = 2.0 ** -10 * (4 * want.abs() + y.abs()) + 1e-4
+    else:
+        want = y + (other.double() if kind == "residual" else 0)
+        tol = 2.0 ** -10 * (y.abs() + want.abs()) + 1e-4
+    assert ((out[:M].double() - want).abs() <= tol).all()
+    assert bool((out[M] == 7.0).all())
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("kind", ["plain", "residual", "gate", "gated", "norm", "norm_gated"])
 @pytest.mark.parametrize("K,N,M", [(64, 64, 1), (512, 128, 16), (1088, 64, 9), (1088, 2560, 8), (4096, 4096, 7), (5120, 5120, 3),
                                    (2048, 8192, 13), (5120, 13696, 12), (64, 65536, 2)])
