@@ -27,8 +27,32 @@ __all__ = ["MetaDesc", "LlamaMmha", "BaichuanMmha", "GatedFeedForwardNetworkInt8
            "deferred_epilogue", "check_device_status", "EETError"]
 
 
+# The raw handle of the current device's current stream, without building a Stream object around it (0.2 us instead of
+# 1.3 us, several times per op).
+_raw_stream = torch._C._cuda_getCurrentRawStream
+_current_device = torch._C._cuda_getDevice
+
+
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
+
+
+class _NoGuard:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_no_guard = _NoGuard()
+
+
+def _on(device):
+    """torch.cuda.device(device), or nothing where that device is current already (the usual case)."""
+    if device.index is None or (torch.cuda.is_initialized() and device.index == _current_device()):
+        return _no_guard
+    return torch.cuda.device(device)
 
 
 def _ptr(t):
@@ -46,8 +70,22 @@ def _ptr(t):
 class _Pool:
     def __init__(self):
         self.buffers = {}
+        self.views = {}
         self.gemm_ws = {}
         self.step_arena = {}
+
+    def rows(self, name, rows, cols, capacity, dtype, device):
+        """The first rows x cols values of get(name, capacity, ...) as a matrix.  The view is kept (a decode step asks for
+        the same ones again and again); callers hand out views of it, never the object itself."""
+        key = (name, rows, cols, dtype, device)
+        view = self.views.get(key)
+        if view is None or capacity > view[1]:
+            if len(self.views) >= 256:
+                self.views.clear()
+            buf = self.get(name, capacity, dtype, device)
+            view = (buf[: rows * cols].view(rows, cols), buf.numel())
+            self.views[key] = view
+        return view[0]
 
     def get(self, name, numel, dtype, device):
         key = (name, str(device), dtype)
@@ -55,6 +93,7 @@ class _Pool:
         if buf is None or buf.numel() < numel:
             buf = torch.empty(max(int(numel), 1), dtype=dtype, device=device)
             self.buffers[key] = buf
+            self.views.clear()   # views of the buffer it replaces
         return buf
 
     def zeros(self, name, numel, dtype, device):
@@ -69,7 +108,7 @@ class _Pool:
 
     def gemm_workspace(self, nbytes, device):
         """Zero-initialised split-K scratch; the GEMM leaves it zero after every call."""
-        key = str(device)
+        key = device
         buf = self.gemm_ws.get(key)
         if buf is None or buf.numel() < nbytes:
             buf = torch.zeros(int(nbytes), dtype=torch.uint8, device=device)
@@ -91,6 +130,7 @@ class _Pool:
 
     def clear(self):
         self.buffers.clear()
+        self.views.clear()
         self.gemm_ws.clear()
 
     def rezero(self):
@@ -248,6 +288,8 @@ def gemm_w8a16(x, packed_w, scale, out=None, residual=None, gate=None):
         out = torch.empty((M, N), dtype=torch.float16, device=x.device)
     if gate is not None and residual is not None:
         raise RuntimeError("gemm_w8a16: residual and gate exclude each other")
+    if M <= _ROW_MAX_M and gate is None and (residual is None or residual.numel() > 0) and M > 0:
+        return _gemm_row(x, packed_w, scale, out, M, residual=residual)
     second, epilogue = (gate, 2) if gate is not None else (residual, 1 if residual is not None else 0)
     ws_bytes = lib.eet_gemm_w8a16_workspace_bytes(M, N, K)
     ws = _pool.gemm_workspace(ws_bytes, x.device)
@@ -535,9 +577,9 @@ class _MmhaBase:
         """Output projection + residual (LlamaMmha::project, llama_mmha.cpp:428-469: the residual is added
         whatever add_residual says)."""
         d = self.desc
-        out = _pool.get("self_mask_attn_cache", d.batch_size * d.max_seq_len * d.hidden_units, torch.float16, d.device)
-        out = out[: B * S * d.hidden_units].view(B * S, d.hidden_units)
-        inp2d = inp.reshape(B * S, d.hidden_units)
+        out = _pool.rows("self_mask_attn_cache", B * S, d.hidden_units, d.batch_size * d.max_seq_len * d.hidden_units,
+                         torch.float16, d.device)
+        inp2d = inp.view(B * S, d.hidden_units)
         _pending.pop(out.data_ptr(), None)   # whatever this buffer held before is gone
         if _row_chain(B * S, d):
             _project_row(ctx2d, self.out_w, self.out_s, out, inp2d, B * S, d, "self_mask_attn_cache")
@@ -576,7 +618,7 @@ class _MmhaBase:
         accepted and ignored exactly as the reference ignores them: the norm always comes first and the
         residual is always added."""
         self._check_input(input)
-        with torch.cuda.device(self.desc.device):
+        with _on(self.desc.device):
             if first_pass:
                 return self._forward_full(input, pre_padding_len, relative_attention_bias)
             return self._forward_inc(input, pre_padding_len, reorder_state, relative_attention_bias)
@@ -591,15 +633,14 @@ class _MmhaBase:
         H, D = d.head_num, self.size_per_head
         M = B * S
         cap = d.batch_size * d.max_seq_len
-        xn = _pool.get("layernorm", cap * h, torch.float16, d.device)[: M * h].view(M, h)
+        xn = _pool.rows("layernorm", M, h, cap * h, torch.float16, d.device)
         _norm_head(inp.view(M, h), self.ln_w, d.layernorm_eps, xn)
-        qkv = _pool.get("qkv_full", cap * 3 * self.inner_dim, torch.float16, d.device)[: M * 3 * self.inner_dim]
-        qkv = qkv.view(M, 3 * self.inner_dim)
+        qkv = _pool.rows("qkv_full", M, 3 * self.inner_dim, cap * 3 * self.inner_dim, torch.float16, d.device)
         _linear(xn, self.qkv_w, self.qkv_s, qkv)
-        q = _pool.get("q_buf", cap * self.inner_dim, torch.float16, d.device)[: M * self.inner_dim]
+        q = _pool.rows("q_buf", M, self.inner_dim, cap * self.inner_dim, torch.float16, d.device)
         check(lib.eet_qkv_split_store(qkv.data_ptr(), q.data_ptr(), self.k_cache.data_ptr(), self.v_cache.data_ptr(),
                                       B, S, H, D, d.max_full_seq_len, int(self.ROPE), self.rope_base, _stream()))
-        ctx = _pool.get("dst", cap * self.inner_dim, torch.float16, d.device)[: M * self.inner_dim]
+        ctx = _pool.rows("dst", M, self.inner_dim, cap * self.inner_dim, torch.float16, d.device)
         alibi = None
         if not self.ROPE:
             if bias is None or bias.numel() == 0:
@@ -609,7 +650,7 @@ class _MmhaBase:
             alibi = bias
         check(lib.eet_prefill_mha(q.data_ptr(), self.k_cache.data_ptr(), self.v_cache.data_ptr(), ctx.data_ptr(),
                                   B, S, H, D, d.max_full_seq_len, _ptr(pre_padding_len), _ptr(alibi), S, _stream()))
-        out = self._project(ctx.view(M, self.inner_dim), inp, B, S)
+        out = self._project(ctx, inp, B, S)
         self.step_ = S
         return out
 
@@ -626,11 +667,10 @@ class _MmhaBase:
         qkv, qkv_sums = None, None
         norm = _take_squares(x2d, self.ln_w, d)
         if norm is None:
-            xn = _pool.get("layernorm_inc", d.batch_size * h, torch.float16, d.device)[: B * h].view(B, h)
+            xn = _pool.rows("layernorm_inc", B, h, d.batch_size * h, torch.float16, d.device)
             _norm_head(x2d, self.ln_w, d.layernorm_eps, xn)
         if norm is not None:
-            qkv = _pool.get("qkv_inc", d.batch_size * 3 * self.inner_dim, torch.float16, d.device)
-            qkv = qkv[: B * 3 * self.inner_dim].view(B, 3 * self.inner_dim)
+            qkv = _pool.rows("qkv_inc", B, 3 * self.inner_dim, d.batch_size * 3 * self.inner_dim, torch.float16, d.device)
             _gemm_row(x2d, self.qkv_w, self.qkv_s, qkv, B, norm=norm)
         elif _defer_ok(B, d):
             # the attention kernel finishes the projection itself: fp16(sums * scale)
@@ -638,12 +678,11 @@ class _MmhaBase:
             qkv_sums = qkv_sums[: B * 3 * self.inner_dim].view(B, 3 * self.inner_dim)
             gemm_w8a16_accum(xn, self.qkv_w, qkv_sums)
         else:
-            qkv = _pool.get("qkv_inc", d.batch_size * 3 * self.inner_dim, torch.float16, d.device)
-            qkv = qkv[: B * 3 * self.inner_dim].view(B, 3 * self.inner_dim)
+            qkv = _pool.rows("qkv_inc", B, 3 * self.inner_dim, d.batch_size * 3 * self.inner_dim, torch.float16, d.device)
             _linear(xn, self.qkv_w, self.qkv_s, qkv)
         if reorder_state is not None and reorder_state.numel() != 0:
             self._reorder(reorder_state, B)
-        ctx = _pool.get("context_buf", d.batch_size * self.inner_dim, torch.float16, d.device)[: B * self.inner_dim]
+        ctx = _pool.rows("context_buf", B, self.inner_dim, d.batch_size * self.inner_dim, torch.float16, d.device)
         alibi, alibi_stride, slopes = None, 0, None
         if not self.ROPE:
             if self.use_device_step:
@@ -662,7 +701,7 @@ class _MmhaBase:
                                  B, H, D, d.max_full_seq_len, self.step_, step_dev, _ptr(pre_padding_len),
                                  _ptr(alibi), alibi_stride, _ptr(slopes), int(self.ROPE), self.rope_base, 0,
                                  _stream()))
-        return self._project(ctx.view(B, self.inner_dim), inp, B, 1)
+        return self._project(ctx, inp, B, 1)
 
     def _reorder(self, reorder_state, B):
         """Beam search: reorder the cache rows first, as LlamaMmha::forward_inc does
@@ -748,14 +787,14 @@ class GatedFeedForwardNetworkInt8:
         B, S, h = input.shape
         M = B * S
         cap = d.batch_size * d.max_seq_len
-        with torch.cuda.device(d.device):
+        with _on(d.device):
             x2d = input.view(M, h)
             norm = _take_squares(x2d, self.ln_w, d)
             if norm is None:
-                xn = _pool.get("layernorm_tensor", cap * h, torch.float16, d.device)[: M * h].view(M, h)
+                xn = _pool.rows("layernorm_tensor", M, h, cap * h, torch.float16, d.device)
                 _norm_head(x2d, self.ln_w, d.layernorm_eps, xn)
-            act = _pool.get("ffn_inner_act", cap * self.d_ff, torch.float16, d.device)[: M * self.d_ff].view(M, self.d_ff)
-            out = _pool.get(self.cache_name, cap * h, torch.float16, d.device)[: M * h].view(M, h)
+            act = _pool.rows("ffn_inner_act", M, self.d_ff, cap * self.d_ff, torch.float16, d.device)
+            out = _pool.rows(self.cache_name, M, h, cap * h, torch.float16, d.device)
             inp2d = x2d
             _pending.pop(out.data_ptr(), None)   # whatever this buffer held before is gone
             deferred = _defer_ok(M, d)
@@ -875,7 +914,7 @@ class LayerNorm:
     def layer_norm(self, input_tensor):
         B, S, h = input_tensor.shape
         out = self.output.view(-1)[: B * S * h].view(B * S, h)
-        with torch.cuda.device(self.desc.device):
+        with _on(self.desc.device):
             _norm_head(input_tensor.reshape(B * S, h), self.gamma, self.desc.layernorm_eps, out)
         return out.view(B, S, h)
 

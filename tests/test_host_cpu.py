@@ -136,3 +136,15 @@ def test_vocab_range_covers_the_vocabulary_in_whole_tiles():
         tp.vocab_range(32001, 0, 2)
     with pytest.raises(ValueError):
         tp.vocab_range(128, 0, 4)
+
+
+def test_pool_rows_follow_a_replaced_buffer():
+    from eet_b200.EET import _Pool
+    pool, dev = _Pool(), torch.device("cpu")
+    a = pool.rows("x", 2, 8, 32, torch.float16, dev)
+    assert pool.rows("x", 2, 8, 32, torch.float16, dev) is a and a.shape == (2, 8)
+    b = pool.rows("x", 4, 16, 64, torch.float16, dev)      # larger: the buffer is replaced, and the kept view with it
+    c = pool.rows("x", 2, 8, 32, torch.float16, dev)
+    assert c.data_ptr() == b.data_ptr() != a.data_ptr()
+    pool.clear()
+    assert pool.rows("x", 2, 8, 32, torch.float16, dev).data_ptr() != 0 and not pool.gemm_ws
