@@ -49,6 +49,7 @@ static inline bool aligned16(const void* p)
 #include "gemm_row.cu"
 #include "gemm_tc.cu"
 #include "gemm_mid.cu"
+#include "gemm_pair.cu"
 #include "attention_tc.cu"
 #include "glue.cu"
 #include "noalloc.cu"
@@ -232,10 +233,18 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
         r.gate = gate;
         return launch_gemm_row(r, (cudaStream_t)stream);
     }
-    // Above 64 tokens two kernels take most shapes: tiles with the epilogue fused, and stream-K units into the fp32 scratch
-    // with a finishing launch.  The shorter modelled time decides (measured on both sides of the line: 4096 x 11008, M = 256:
-    // tiles 28 us, units 37; 13696 x 5120, M = 256: 52 and 42).
-    const bool tiles_first = M > 64 && gemm_tc_us(M, N, K) < gemm_mid_us(M, N, K);
+    // Above 64 tokens three kernels take most shapes: tiles on single CTAs or on CTA pairs, both with the epilogue fused, and
+    // stream-K units into the fp32 scratch with a finishing launch.  The shortest modelled time decides (measured on both
+    // sides of the lines: 4096 x 11008, M = 256: tiles 28 us, units 37; 13696 x 5120, M = 256: 52 and 42; M = 4096 on
+    // 11008 x 4096: single CTAs 267, pairs 249; 4096 x 12288, M = 512: 50 and 59).
+    const double tc_us = M > 64 ? gemm_tc_us(M, N, K) : 1e30;
+    const PairPlan pair = gemm_pair_plan(M, N, K);
+    const double mid_us = M <= mid_use_max_m() ? gemm_mid_us(M, N, K) : 1e30;
+    if (pair.bn > 0 && pair.us < tc_us && pair.us < mid_us) {
+        return launch_gemm_pair((const __half*)A, (const uint8_t*)packedB, (const __half*)scale, (__half*)C, res, gate, M, N, K,
+                                pair.bn, (cudaStream_t)stream);
+    }
+    const bool tiles_first = M > 64 && tc_us < mid_us;
     if (!tiles_first && M <= mid_use_max_m() && gemm_mid_supported(M, N, K)) {
         // stream-K tensor-core kernel into the fp32 scratch, then one epilogue pass over all rows
         EET_CHECK(ws && aligned16(ws) && ws_bytes >= skinny_sum_bytes(M, N),

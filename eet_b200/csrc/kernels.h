@@ -54,6 +54,15 @@ double gemm_tc_us(int M, int N, int K);  // modelled time in microseconds (large
 int launch_gemm_tc(const __half* A, const uint8_t* B, const __half* scale, __half* C, const __half* residual, int gate,
                    int M, int N, int K, cudaStream_t stream);
 
+// gemm_pair.cu (tcgen05 on CTA pairs)
+struct PairPlan {
+    int bn;       // tokens per accumulator; 0: the kernel does not take the shape
+    double us;    // modelled time in microseconds
+};
+PairPlan gemm_pair_plan(int M, int N, int K);
+int launch_gemm_pair(const __half* A, const uint8_t* B, const __half* scale, __half* C, const __half* residual, int gate,
+                     int M, int N, int K, int bn, cudaStream_t stream);
+
 // gemm_mid.cu (stream-K tcgen05, fp32 sums like the skinny kernel)
 constexpr int kMidMaxM = 512;
 bool gemm_mid_supported(int M, int N, int K);

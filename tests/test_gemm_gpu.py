@@ -112,10 +112,12 @@ def test_empty_and_invalid():
 
 @pytest.mark.parametrize("kind", ["plain", "residual", "gate"])
 @pytest.mark.parametrize("K,N,M", [(64, 128, 65), (320, 384, 97), (1024, 640, 513), (4096, 4224, 130), (640, 13696, 999),
-                                   (2048, 896, 4095), (5120, 256, 700), (13696, 5120, 600), (192, 38016, 259)])
+                                   (2048, 896, 4095), (5120, 256, 700), (13696, 5120, 600), (192, 38016, 259),
+                                   (1024, 13696, 2049), (1152, 2176, 1813), (1280, 1152, 3434), (960, 12928, 1319),
+                                   (3264, 11392, 4006)])
 def test_prefill_gemm_tiles(K, N, M, kind):
     """Tiles with a lower half only, token tiles that are no multiple of 32, whole waves, waves with a split remainder and
-    split tiles only, few k-blocks.  Bound: fp32 sums, one fp16 rounding of the product and one of the sum with the
+    split tiles only, tiles on CTA pairs (several per pair, one wave, no upper half), few k-blocks.  Bound: fp32 sums, one fp16 rounding of the product and one of the sum with the
     residual, 2^-11 each, doubled; the activation's error is its operands' plus its own three fp16 steps."""
     from eet_b200 import EET, _lib
     gen = torch.Generator(device="cuda").manual_seed(M)
