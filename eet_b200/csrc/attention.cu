@@ -34,7 +34,7 @@ constexpr int kHalfWarps = kAttnConsumerThreads / 16;
 #ifndef EET_ATTN_TILE
 #define EET_ATTN_TILE 32
 #define EET_ATTN_STAGES 2
-#define EET_ATTN_CTAS 5
+#define EET_ATTN_CTAS 4
 #endif
 constexpr int kAttnTile = EET_ATTN_TILE;                     // time steps per shared-memory stage
 constexpr int kAttnStages = EET_ATTN_STAGES;
@@ -104,8 +104,10 @@ struct AttnSmem {
 //
 // Data path: the history slice of a CTA is contiguous in the [B][H][T][D] caches, so a producer warp
 // streams it with 1-D bulk copies (TMA engine) of 32 time steps of K and of V per stage into a two-stage
-// ring; five CTAs per SM keep ~160 KiB in flight.  Register-level loads of the same bytes stall on the
-// number of outstanding L1 misses long before HBM is busy.  Four consumer warps take a half-warp per time
+// ring; four CTAs per SM keep ~128 KiB in flight, and 96 registers a thread hold a tile's K and V pieces (with five CTAs the
+// 72 registers left spilled: the op at 8 x 1000 tokens 46.0 us, now 42.9; a decode step of 4 layers 269.8, now 259.9; three
+// CTAs leave room for no split of a history at 8 x 32 heads: 49.3 and 271.6).  Register-level loads of the same bytes stall
+// on the number of outstanding L1 misses long before HBM is busy.  Four consumer warps take a half-warp per time
 // step from shared memory.
 __global__ void __launch_bounds__(kAttnThreads, kAttnCtasPerSm)
 decode_mha_kernel(DecodeAttnArgs a)
@@ -623,7 +625,7 @@ int launch_decode_mha(const DecodeAttnArgs& a, cudaStream_t stream)
     if (a.B == 0) return 0;
     int splits = a.splits;
     if (splits == 0) {
-        // as many CTAs as fit on the machine at once (5 per SM); at least 64 time steps per CTA
+        // as many CTAs as fit on the machine at once (four per SM); at least 64 time steps per CTA
         const int len = a.step_dev ? a.T_max : a.step;
         const int room = kAttnCtasPerSm * sm_count() / (a.B * a.H);
         splits = 1;
