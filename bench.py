@@ -630,7 +630,7 @@ def run_ours(args):
                          "frac": round(dom["gbs"] / pk["hbm_gbs"], 4), "peak_source": pk["source"],
                          "traffic": None if traffic is None else round(traffic),
                          "traffic_source": None if traffic is None else
-                         "not measured by this run: one ncu capture of this kernel at K=4096 N=12288 M=8 "
+                         "not measured by this run: one ncu capture of the accumulate kernel at K=4096 N=12288 M=8 "
                          "(50.81 MB read+written for 50.62 MB algorithmic), scaled by this launch's algorithmic bytes",
                          "algorithmic_bytes": dom["bytes"],
                          "launch_us": round(dom["us"], 2),
