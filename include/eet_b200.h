@@ -63,7 +63,7 @@ size_t eet_quantize_w8_workspace_bytes(int K, int N);
  *   packed       device, K*N bytes in the W8T64 layout consumed by eet_gemm_w8a16
  *   scales       device [N], fp16 when w is fp16, fp32 when w is fp32
  *   variant      0 = reference (amax/128, clip [-128,127]); 1 = amax/127, clip [-127,127]
- *   ws           device scratch of eet_quantize_w8_workspace_bytes(K, N) bytes
+ *   ws           device scratch of eet_quantize_w8_workspace_bytes(K, N) bytes, aligned to 4 bytes
  */
 int eet_quantize_w8(const void* w, int w_is_fp32, int K, int N, int8_t* q_rowmajor, void* packed, void* scales,
                     int variant, void* ws, size_t ws_bytes, void* stream);

@@ -93,6 +93,23 @@ def test_variant_127_and_three_d_input():
     assert int(q.min()) >= -127
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("offset", [4, 8, 12])
+def test_quantizer_scratch_needs_no_more_than_float_alignment(dtype, offset):
+    """A scratch that begins anywhere in a larger allocation of the caller: the same bits, its neighbours untouched."""
+    from eet_b200 import EET
+    from eet_b200._lib import check, lib
+    K, N = 192, 320
+    w = (torch.randn(K, N, generator=torch.Generator().manual_seed(offset)) * 0.02).to(dtype).cuda()
+    packed, scales = EET.quant_weights(w, torch.int8)
+    ws = torch.full((N + 8,), -3.0, device="cuda")
+    p2, s2 = torch.zeros_like(packed), torch.zeros_like(scales)
+    check(lib.eet_quantize_w8(w.data_ptr(), int(dtype == torch.float32), K, N, None, p2.data_ptr(), s2.data_ptr(), 0,
+                              ws.data_ptr() + offset, 4 * N, torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(p2, packed) and torch.equal(_bits(s2), _bits(scales))
+    assert bool((ws[: offset // 4] == -3.0).all()) and bool((ws[offset // 4 + N:] == -3.0).all())
+
+
 def test_cuda_input_stays_on_device_and_bad_shapes_raise():
     from eet_b200 import EET
     w = torch.randn(64, 128, device="cuda").half()
