@@ -249,7 +249,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __re
             const int n0 = (tile % tiles_n) * 256;
             const bool mine = n0 + rank * 128 < N;
             for (int kb = 0; kb < KT; ++kb, ++it) {
-                if (!tc_wait(&sm.w_full[sw], phw, &sm.abort)) {
+                if (!tc_wait_warp(&sm.w_full[sw], phw, &sm.abort)) {
                     ok = false;
                     break;
                 }
@@ -270,7 +270,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __re
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sm.w_empty[sw]);
                 if (it >= kPrNH) {
-                    if (!tc_wait(&sm.done[d], phd, &sm.abort)) {
+                    if (!tc_wait_warp(&sm.done[d], phd, &sm.abort)) {
                         ok = false;
                         break;
                     }
@@ -297,11 +297,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __re
                     phw ^= 1;
                 }
             }
-            if (!ok) break;
 
-            // ---- end of the tile: every epilogue warp gets here (the waits are bounded); the OR-reducing
-            // barrier gives all 256 epilogue threads the same answer, whoever saw the abort flag first ----
-            tc_wait(&sm.accum, (uint32_t)(p & 1), &sm.abort);
+            // ---- end of the tile: every epilogue warp gets here, also one that has left the loop above because a wait ran out
+            // (the others may have finished theirs); the OR-reducing barrier gives all 256 epilogue threads the same answer,
+            // whoever saw the abort flag first ----
+            if (ok) tc_wait_warp(&sm.accum, (uint32_t)(p & 1), &sm.abort);
             if (epi_bar_or(sm.abort != 0)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             pdl_wait();   // the output and the residual belong to the dependency chain

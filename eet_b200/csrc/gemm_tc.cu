@@ -59,6 +59,25 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile
     return tc_wait_slow(bar, parity, abort);
 }
 
+// The same for the 32 lanes of a converged warp: all of them get the same answer, so the warp cannot part on its way to a
+// barrier.  (One vote where the phase is complete already, the usual case.)
+__device__ __noinline__ bool tc_wait_warp_slow(uint64_t* bar, uint32_t parity, volatile int* abort)
+{
+    for (uint32_t i = 0; i < kTcSpin; ++i) {
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        if (__any_sync(0xffffffffu, *abort)) return false;
+    }
+    *abort = 1;
+    g_device_status = 2;
+    return false;
+}
+
+__device__ __forceinline__ bool tc_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort)
+{
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    return tc_wait_warp_slow(bar, parity, abort);
+}
+
 // shared-memory matrix descriptor: K-major, 128-byte swizzle, rows of 128 bytes, 8-row groups 1024 B apart
 __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr)
 {
@@ -457,7 +476,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
             const Tc2Seg sg = wk.seg(p);
             const bool mine = grp == 0 || (sg.tile % tiles_n) * 256 + 128 < N;   // (the last tile may have no upper half)
             for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
-                if (!tc_wait(&sm.w_full[sw], phw, &sm.abort)) {
+                if (!tc_wait_warp(&sm.w_full[sw], phw, &sm.abort)) {
                     ok = false;
                     break;
                 }
@@ -481,7 +500,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sm.w_empty[sw]);
                 if (it >= kTc2NH) {
-                    if (!tc_wait(&sm.done[d], phd, &sm.abort)) {
+                    if (!tc_wait_warp(&sm.done[d], phd, &sm.abort)) {
                         ok = false;
                         break;
                     }
@@ -510,11 +529,11 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
                     phw ^= 1;
                 }
             }
-            if (!ok) break;
 
-            // ---- end of the segment: every epilogue warp gets here (the waits are bounded); the OR-reducing
-            // barrier gives all 256 epilogue threads the same answer, whoever saw the abort flag first ----
-            tc_wait(&sm.accum, (uint32_t)(p & 1), &sm.abort);
+            // ---- end of the segment: every epilogue warp gets here, also one that has left the loop above because a wait ran
+            // out (the others may have finished theirs); the OR-reducing barrier gives all 256 epilogue threads the same
+            // answer, whoever saw the abort flag first ----
+            if (ok) tc_wait_warp(&sm.accum, (uint32_t)(p & 1), &sm.abort);
             if (epi_bar_or(sm.abort != 0)) {
                 ok = false;
                 break;

@@ -1,0 +1,32 @@
+"""Rules of the kernels' source that no run can show without a hang or a race: read from the text."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "eet_b200", "csrc")
+
+
+def _source(name):
+    return re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+
+
+@pytest.mark.parametrize("name", ["gemm_tc.cu", "gemm_pair.cu"])
+def test_warps_whose_wait_ran_out_join_the_barrier_of_the_epilogue(name):
+    """Between a tile's loop over its k-blocks and epi_bar_or, a barrier that counts all 256 threads of the transform
+    warps, nothing may leave: a warp that gives up there would keep the warps that finished their loop waiting for ever.
+    And the waits in that loop answer a whole warp alike, so that no warp arrives in two parts."""
+    text = _source(name)
+    role = text[text.index("const int lane_base = (warp & 3) * 32;"):]
+    at = role.index("epi_bar_or(")
+    depth, body_end = 0, None
+    start = role.index("{", role.index("for (int kb = "))
+    for i in range(start, at):
+        depth += {"{": 1, "}": -1}.get(role[i], 0)
+        if depth == 0:
+            body_end = i
+            break
+    assert body_end is not None, "the loop over the k-blocks encloses the barrier"
+    assert not re.search(r"\b(break|return|continue|goto)\b", role[body_end:at])
+    waits = re.findall(r"\btc_wait\w*\(", role[start:at])
+    assert len(waits) == 3 and set(waits) == {"tc_wait_warp("}
