@@ -239,16 +239,19 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
     // 11008 x 4096: single CTAs 267, pairs 249; 4096 x 12288, M = 512: 50 and 59).
     const double tc_us = M > 64 ? gemm_tc_us(M, N, K) : 1e30;
     const PairPlan pair = gemm_pair_plan(M, N, K);
-    const double mid_us = M <= mid_use_max_m() ? gemm_mid_us(M, N, K) : 1e30;
+    const bool sums_allowed = M <= mid_use_max_m() && gemm_mid_supported(M, N, K) && !gemm_tc_owns(M, N, K);
+    if (sums_allowed) {
+        // (asked for whichever kernel is chosen: whether a caller has to bring scratch hangs on the shape alone)
+        EET_CHECK(ws && aligned16(ws) && ws_bytes >= skinny_sum_bytes(M, N),
+                  "eet_gemm_w8a16: workspace of %zu bytes is smaller than the %zu needed", ws_bytes, skinny_sum_bytes(M, N));
+    }
+    const double mid_us = sums_allowed ? gemm_mid_us(M, N, K) : 1e30;
     if (pair.bn > 0 && pair.us < tc_us && pair.us < mid_us) {
         return launch_gemm_pair((const __half*)A, (const uint8_t*)packedB, (const __half*)scale, (__half*)C, res, gate, M, N, K,
                                 pair.bn, (cudaStream_t)stream);
     }
-    const bool tiles_first = M > 64 && tc_us < mid_us;
-    if (!tiles_first && M <= mid_use_max_m() && gemm_mid_supported(M, N, K)) {
+    if (sums_allowed && !(M > 64 && tc_us < mid_us)) {
         // stream-K tensor-core kernel into the fp32 scratch, then one epilogue pass over all rows
-        EET_CHECK(ws && aligned16(ws) && ws_bytes >= skinny_sum_bytes(M, N),
-                  "eet_gemm_w8a16: workspace of %zu bytes is smaller than the %zu needed", ws_bytes, skinny_sum_bytes(M, N));
         GemmArgs a = {};
         a.A = (const __half*)A;
         a.B = (const uint8_t*)packedB;

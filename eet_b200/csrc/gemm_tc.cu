@@ -765,6 +765,20 @@ bool gemm_tc_supported(int M, int N, int K)
     return M >= kTcMinM && N % 128 == 0 && K % 64 == 0;
 }
 
+// Shapes that always go to tiles, whatever the models say: enough channels for 120 tiles of 256 x 256, or for 96 CTAs once
+// their k-blocks are split over the largest cluster that fits.  A caller may rely on it: such a call needs no scratch and
+// gives the same bits every time, which the stream-K kernel, whose sums meet in the order of arrival, does not.
+bool gemm_tc_owns(int M, int N, int K)
+{
+    if (M < kTcMinM || N % 256 != 0) return false;
+    const long long tiles = (long long)(N / 256) * ((M + 255) / 256);
+    if (tiles >= 120) return true;
+    for (int sp = 4; sp >= 2; --sp) {
+        if (K / kTile / sp >= 4 && tiles <= tc2_max_clusters(sp)) return tiles * sp >= 96;
+    }
+    return false;
+}
+
 // Modelled time in microseconds; a large number where the kernel does not take the shape.
 double gemm_tc_us(int M, int N, int K)
 {

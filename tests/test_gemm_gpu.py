@@ -266,6 +266,33 @@ def test_baichuan13b_and_llama65b_projection_shapes(KN):
     assert ((y[rows].double() - ref).abs() <= 1e-2 * ref.abs().amax(1, keepdim=True)).all()
 
 
+@pytest.mark.parametrize("K,N,M", [(4096, 11008, 65), (4096, 11008, 100), (4096, 12288, 128), (8192, 8192, 80),
+                                   (5120, 5120, 384), (8192, 3072, 512), (1088, 6144, 300)])
+def test_wide_shapes_repeat_bit_for_bit_and_need_no_scratch(K, N, M):
+    """From 65 rows on, shapes with enough 256-channel tiles (whole, or split over clusters): the same bits every time, and no
+    scratch.  Narrow ones sum in global memory: without scratch they are refused."""
+    from eet_b200._lib import check, lib
+    from eet_b200 import EET
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    q = torch.randint(-127, 128, (K, N), generator=gen, device="cuda", dtype=torch.int8)
+    s = ((torch.rand(N, generator=gen, device="cuda") + 0.5) * K ** -0.5 / 64).half()
+    x = torch.randn(M, K, generator=gen, device="cuda").half()
+    packed = EET.preprocess_weights(q)
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def call(w, n):
+        out = torch.empty(M, n, dtype=torch.float16, device="cuda")
+        rc = lib.eet_gemm_w8a16(x.data_ptr(), w.data_ptr(), s.data_ptr(), out.data_ptr(), M, n, K, None, 0, None, 0, stream)
+        return rc, out
+    rc, first = call(packed, N)
+    check(rc)
+    y = (x.double() @ q.double()) * s.double()
+    assert ((first.double() - y).abs() <= 2.0 ** -10 * y.abs() + 1e-4).all()   # one rounding to fp16, doubled
+    for _ in range(8):
+        assert torch.equal(call(packed, N)[1], first)
+    assert call(EET.preprocess_weights(q[:, :128].contiguous()), 128)[0] != 0 and b"workspace" in lib.eet_last_error()
+
+
 @pytest.mark.parametrize("M", [17, 32, 40, 64, 100, 128, 250, 256, 400, 512])
 @pytest.mark.parametrize("KN", [(256, 128), (192, 256), (1024, 384), (4096, 4096)])
 def test_stream_k_tensor_core_kernel(KN, M):
