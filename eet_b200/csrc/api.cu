@@ -205,6 +205,53 @@ int eet_gemm_w8a16_finalize(float* sums, const void* scale, const void* residual
     return launch_finalize(sums, (const __half*)scale, (const __half*)residual, (__half*)C, M, N, (cudaStream_t)stream);
 }
 
+// Which kernel a shape goes to.  Up to 16 rows the row kernel.  Above that stream-K units into fp32 scratch with a finishing
+// launch, tiles on single CTAs or tiles on CTA pairs, both with the epilogue fused: the shortest modelled time decides, among
+// those that the shape may take.  Measured on both sides of the lines: 4096 x 4096, M = 128 units 15 us, tiles 18, and at M = 256
+// 21.7 and 20.2; 4096 x 32000, M = 384 units 148, tiles 100, pairs 94; 11008 x 4096, M = 4096 single CTAs 267, pairs 249.
+enum { kRouteShares = 0, kRouteRow = 1, kRouteStreamK = 2, kRouteTiles = 3, kRoutePairs = 4 };
+
+struct GemmRoute {
+    int kernel;
+    bool scratch;     // a caller has to bring the fp32 sums: hangs on the shape alone, whichever kernel is chosen
+    Tc2Plan tc;
+    PairPlan pair;
+};
+
+static GemmRoute gemm_route(int M, int N, int K)
+{
+    GemmRoute r = {kRouteShares, true, Tc2Plan{0, 0, 0, 1, 1e30}, PairPlan{0, 1e30}};
+    if (M <= kRowMaxM) {
+        r.kernel = kRouteRow;
+        return r;
+    }
+    const bool sums = M <= mid_use_max_m() && gemm_mid_supported(M, N, K) && !gemm_tc_owns(M, N, K);
+    double least = sums ? gemm_mid_us(M, N, K) : 1e30;
+    if (sums) r.kernel = kRouteStreamK;
+    r.tc = gemm_tc_plan(M, N, K);
+    r.pair = gemm_pair_plan(M, N, K);
+    if (r.tc.us < least) {
+        r.kernel = kRouteTiles;
+        least = r.tc.us;
+    }
+    if (r.pair.us < least) r.kernel = kRoutePairs;
+    r.scratch = sums || r.kernel == kRouteShares;
+    return r;
+}
+
+int eet_gemm_w8a16_plan(int M, int N, int K, int* plan)
+{
+    if (check_kn("eet_gemm_w8a16_plan", K, N)) return 1;
+    EET_CHECK(M > 0 && plan != nullptr, "eet_gemm_w8a16_plan: M must be positive and plan not NULL");
+    const GemmRoute r = gemm_route(M, N, K);
+    plan[0] = r.kernel;
+    plan[1] = r.kernel == kRouteTiles ? r.tc.bn : (r.kernel == kRoutePairs ? 2 * r.pair.bn : 0);
+    plan[2] = r.kernel == kRouteTiles ? r.tc.whole : 0;
+    plan[3] = r.kernel == kRouteTiles ? r.tc.tiles - r.tc.whole : 0;
+    plan[4] = r.kernel == kRouteTiles ? r.tc.split : 0;
+    return 0;
+}
+
 int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* C, int M, int N, int K,
                    const void* residual, int epilogue, void* ws, size_t ws_bytes, void* stream)
 {
@@ -216,11 +263,12 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
               "eet_gemm_w8a16: epilogues 1 and 2 need a 16-byte aligned second operand");
     const __half* res = epilogue != 0 ? (const __half*)residual : nullptr;
     const int gate = epilogue == 2 ? 1 : 0;
-    if (M <= kRowMaxM) {
-        // decode regime: one launch, no scratch (the check stays: this entry point has always asked for it)
-        EET_CHECK(ws && aligned16(ws) && ws_bytes >= eet_gemm_w8a16_workspace_bytes(M, N, K),
-                  "eet_gemm_w8a16: workspace of %zu bytes is smaller than the %zu needed", ws_bytes,
-                  eet_gemm_w8a16_workspace_bytes(M, N, K));
+    const GemmRoute route = gemm_route(M, N, K);
+    EET_CHECK(!route.scratch || (ws && aligned16(ws) && ws_bytes >= eet_gemm_w8a16_workspace_bytes(M, N, K)),
+              "eet_gemm_w8a16: workspace of %zu bytes is smaller than the %zu needed", ws_bytes,
+              eet_gemm_w8a16_workspace_bytes(M, N, K));
+    if (route.kernel == kRouteRow) {
+        // decode regime: one launch that leaves the scratch alone (this entry point has always asked for it)
         RowGemmArgs r = {};
         r.A = (const __half*)A;
         r.B = (const uint8_t*)packedB;
@@ -233,45 +281,19 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
         r.gate = gate;
         return launch_gemm_row(r, (cudaStream_t)stream);
     }
-    // Above 64 tokens three kernels take most shapes: tiles on single CTAs or on CTA pairs, both with the epilogue fused, and
-    // stream-K units into the fp32 scratch with a finishing launch.  The shortest modelled time decides (measured on both
-    // sides of the lines: 4096 x 11008, M = 256: tiles 28 us, units 37; 13696 x 5120, M = 256: 52 and 42; M = 4096 on
-    // 11008 x 4096: single CTAs 267, pairs 249; 4096 x 12288, M = 512: 50 and 59).
-    const double tc_us = M > 64 ? gemm_tc_us(M, N, K) : 1e30;
-    const PairPlan pair = gemm_pair_plan(M, N, K);
-    const bool sums_allowed = M <= mid_use_max_m() && gemm_mid_supported(M, N, K) && !gemm_tc_owns(M, N, K);
-    if (sums_allowed) {
-        // (asked for whichever kernel is chosen: whether a caller has to bring scratch hangs on the shape alone)
-        EET_CHECK(ws && aligned16(ws) && ws_bytes >= skinny_sum_bytes(M, N),
-                  "eet_gemm_w8a16: workspace of %zu bytes is smaller than the %zu needed", ws_bytes, skinny_sum_bytes(M, N));
-    }
-    const double mid_us = sums_allowed ? gemm_mid_us(M, N, K) : 1e30;
-    if (pair.bn > 0 && pair.us < tc_us && pair.us < mid_us) {
+    if (route.kernel == kRoutePairs) {
         return launch_gemm_pair((const __half*)A, (const uint8_t*)packedB, (const __half*)scale, (__half*)C, res, gate, M, N, K,
-                                pair.bn, (cudaStream_t)stream);
+                                route.pair.bn, (cudaStream_t)stream);
     }
-    if (sums_allowed && !(M > 64 && tc_us < mid_us)) {
-        // stream-K tensor-core kernel into the fp32 scratch, then one epilogue pass over all rows
-        GemmArgs a = {};
-        a.A = (const __half*)A;
-        a.B = (const uint8_t*)packedB;
-        a.ws = (float*)ws;
-        a.M = M;
-        a.N = N;
-        a.K = K;
-        if (int rc = launch_gemm_mid(a, (cudaStream_t)stream)) return rc;
-        return launch_finalize((float*)ws, (const __half*)scale, res, (__half*)C, M, N, (cudaStream_t)stream, gate);
-    }
-    if (gemm_tc_supported(M, N, K)) {
-        // prefill regime: tcgen05 tensor-core kernel, epilogue fused, no scratch
+    if (route.kernel == kRouteTiles) {
         return launch_gemm_tc((const __half*)A, (const uint8_t*)packedB, (const __half*)scale, (__half*)C, res, gate, M, N,
                               K, (cudaStream_t)stream);
     }
-    EET_CHECK(ws && aligned16(ws) && ws_bytes >= eet_gemm_w8a16_workspace_bytes(M, N, K),
-              "eet_gemm_w8a16: workspace of %zu bytes is smaller than the %zu needed", ws_bytes,
-              eet_gemm_w8a16_workspace_bytes(M, N, K));
-    for (int r0 = 0; r0 < M; r0 += kSkinnyGroupRows) {
-        const int rows = (M - r0 < kSkinnyGroupRows) ? (M - r0) : kSkinnyGroupRows;
+    // sums into the fp32 scratch, then one epilogue pass: all rows at once on the stream-K tensor-core kernel, in groups of
+    // rows on the equal-share kernel
+    const int group = route.kernel == kRouteStreamK ? M : kSkinnyGroupRows;
+    for (int r0 = 0; r0 < M; r0 += group) {
+        const int rows = (M - r0 < group) ? (M - r0) : group;
         GemmArgs a = {};
         a.A = (const __half*)A + (size_t)r0 * K;
         a.B = (const uint8_t*)packedB;
@@ -279,7 +301,8 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
         a.M = rows;
         a.N = N;
         a.K = K;
-        if (int rc = launch_gemm_skinny(a, (cudaStream_t)stream)) return rc;
+        if (int rc = route.kernel == kRouteStreamK ? launch_gemm_mid(a, (cudaStream_t)stream) : launch_gemm_skinny(a, (cudaStream_t)stream))
+            return rc;
         if (int rc = launch_finalize((float*)ws, (const __half*)scale, res ? res + (size_t)r0 * N : nullptr,
                                      (__half*)C + (size_t)r0 * N, rows, N, (cudaStream_t)stream, gate))
             return rc;

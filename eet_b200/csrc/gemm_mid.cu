@@ -429,14 +429,24 @@ bool gemm_mid_supported(int M, int N, int K)
     return M > 16 && M <= kMidMaxM && N % 128 == 0 && K % 64 == 0;
 }
 
-// A fit to measurements at M = 100 ... 512 on the LLaMA-7B and Baichuan-13B shapes (within 8 %): units of 128 channels x 128
-// reduction indices per SM, and 128-token tiles.
+// The token tile of a launch: the smallest that holds M; above 128 tokens 256-token tiles (half the activation traffic per flop,
+// MMAs long enough to hide their issue cost) when every CTA still gets a decent run of units.
+static int mid_bn(int M, long long units)
+{
+    if (M > 128 && units >= 16LL * sm_count()) return 256;
+    return M <= 32 ? 32 : (M <= 64 ? 64 : 128);
+}
+
+// Modelled time with the finishing launch, above 64 rows: per token tile and unit per SM 0.65 us at 128 tokens and 0.86 at 256, and
+// 3.4 ps for each fp32 sum that goes to memory and back.  Fitted to 190 measured times at 65 to 512 rows on 16 weight shapes
+// from 4096 x 1536 to 8192 x 24576, spread 3 %.
 double gemm_mid_us(int M, int N, int K)
 {
     if (!gemm_mid_supported(M, N, K)) return 1e30;
-    const double units = (double)(N / 128) * ((K / kTile + kMidUnitK - 1) / kMidUnitK) / sm_count();
-    const int t = (M + 127) / 128;
-    return 6.0 + 2.9 * t + (0.38 + 0.38 * t) * units;
+    const long long units = (long long)(N / 128) * ((K / kTile + kMidUnitK - 1) / kMidUnitK);
+    const int bn = mid_bn(M, units);
+    const double per_sm = (double)units / sm_count() * ((M + bn - 1) / bn);
+    return (bn == 256 ? 11.5 + 0.86 * per_sm : 8.0 + 0.65 * per_sm) + 3.4e-6 * M * (double)N;
 }
 
 // Adds A[M,K] x q(B) (and, with B2, A x q(B2)) into the fp32 buffers a.ws (a.ws2), rows [0, M).
@@ -451,11 +461,8 @@ int launch_gemm_mid(const GemmArgs& a, cudaStream_t stream)
         const char* e = getenv("EET_MID_BN");
         force_bn = e ? atoi(e) : 0;
     }
-    // token tile: the smallest that holds M; above 128 tokens 256-token tiles (half the activation traffic
-    // per flop, MMAs long enough to hide their issue cost) when every CTA still gets a decent run of units
     const long long units = (long long)(a.N / 128) * ((a.K / kTile + kMidUnitK - 1) / kMidUnitK) * (a.B2 ? 2 : 1);
-    int bn = a.M <= 32 ? 32 : (a.M <= 64 ? 64 : 128);
-    if (a.M > 128 && units >= 16LL * sm_count()) bn = 256;
+    int bn = mid_bn(a.M, units);
     if (force_bn) bn = force_bn;
     CUtensorMap map;
     const cuuint64_t dims[2] = {(cuuint64_t)a.K, (cuuint64_t)a.M};

@@ -712,13 +712,9 @@ static int tc2_max_clusters(int split)
     return cached[dev][split] > 0 ? cached[dev][split] : 0;
 }
 
-// How a shape is run: BN tokens per tile; the first `whole` tiles on persistent CTAs, the others (none, the last partial
-// wave, or all) with their k-blocks split over clusters of `split` CTAs; and the modelled time in microseconds.
-struct Tc2Plan {
-    int bn, tiles, whole, split;
-    double us;
-};
-
+// How a shape is run (Tc2Plan): BN tokens per tile; the first `whole` tiles on persistent CTAs, the others (none, the last partial
+// wave, or all) with their k-blocks split over clusters of `split` CTAs; and the modelled time.
+//
 // Time of a k-block of a 256 x BN tile with the machine full, measured at BN = 64 ... 256 on 4096 x 12288.  Below 128 tokens
 // the conversion of the weights and the hand-overs set the pace, above it the tensor core and shared memory.
 static double tc2_block_us(int bn)
@@ -751,6 +747,9 @@ static Tc2Plan tc2_plan(int M, int N, int K)
             const int left = sp > 1 ? tiles % G : 0, whole = tiles - left;
             if (sp > 1 && (left == 0 || KT / sp < 4 || left > tc2_max_clusters(sp))) continue;
             if (forced >= 0 && sp != 1 && sp != forced) continue;
+            // behind a wave of single CTAs the last few clusters of three find no room until others end and take a second turn
+            // (8192 x 8192, M = 1200, 44 of them: 174 us; 12 clusters of four, BN = 256: 150)
+            if (sp == 3 && whole > 0 && left > 40) continue;
             double us = 5.5 + (double)((whole + G - 1) / G) * (KT * block + epilogue);
             if (left > 0) us += (KT + sp - 1) / sp * block + epilogue + 4.0 + (whole > 0 ? 2.0 : 0.0);
             if (forced == sp && sp > 1 && whole == 0) us *= 0.1;
@@ -779,10 +778,9 @@ bool gemm_tc_owns(int M, int N, int K)
     return false;
 }
 
-// Modelled time in microseconds; a large number where the kernel does not take the shape.
-double gemm_tc_us(int M, int N, int K)
+Tc2Plan gemm_tc_plan(int M, int N, int K)
 {
-    return gemm_tc_supported(M, N, K) ? tc2_plan(M, N, K).us : 1e30;
+    return gemm_tc_supported(M, N, K) ? tc2_plan(M, N, K) : Tc2Plan{0, 0, 0, 1, 1e30};
 }
 
 int launch_gemm_tc(const __half* A, const uint8_t* B, const __half* scale, __half* C, const __half* residual, int gate,

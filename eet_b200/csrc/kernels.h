@@ -51,7 +51,11 @@ int launch_gemm_row(RowGemmArgs a, cudaStream_t stream);
 // gemm_tc.cu (tcgen05 / TMEM)
 bool gemm_tc_supported(int M, int N, int K);
 bool gemm_tc_owns(int M, int N, int K);      // shapes that no kernel with fp32 sums in global memory may take
-double gemm_tc_us(int M, int N, int K);  // modelled time in microseconds (large: the kernel does not take the shape)
+struct Tc2Plan {
+    int bn, tiles, whole, split;   // tokens per tile; tiles; those on single CTAs; CTAs for each of the others
+    double us;                     // modelled time in microseconds (large: the kernel does not take the shape)
+};
+Tc2Plan gemm_tc_plan(int M, int N, int K);
 int launch_gemm_tc(const __half* A, const uint8_t* B, const __half* scale, __half* C, const __half* residual, int gate,
                    int M, int N, int K, cudaStream_t stream);
 

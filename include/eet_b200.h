@@ -116,6 +116,15 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
                    const void* residual, int epilogue, void* ws, size_t ws_bytes, void* stream);
 
 /*
+ * The kernel that eet_gemm_w8a16 gives a shape to on the current device, for tests and tools; launches nothing.
+ *   plan[0]  0 equal shares into the scratch (gemm_skinny.cu), 1 row kernel (gemm_row.cu), 2 stream-K into the scratch
+ *            (gemm_mid.cu), 3 tiles on single CTAs or clusters (gemm_tc.cu), 4 tiles on CTA pairs (gemm_pair.cu)
+ *   plan[1]  tokens per tile (3 and 4)
+ *   plan[2], plan[3], plan[4]  with 3: tiles on single CTAs, tiles whose reduction is split over a cluster, its size
+ */
+int eet_gemm_w8a16_plan(int M, int N, int K, int* plan);
+
+/*
  * The decode GEMM (M <= 16) with what stands around it in a decoder layer, in one launch and without scratch:
  *   gamma, squares_in  both NULL: the activations are A; else they are rmsnorm(A) with weights gamma [K] and eps, the
  *                      norm at the head of a block (csrc/core/layer_norm.cu:490-531); squares_in [M][K/64] fp32 holds

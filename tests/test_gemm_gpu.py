@@ -40,6 +40,37 @@ def _check(y, x, q, s):
     assert ((y.double() - exact).abs() <= 2e-3 * ref.abs().amax(1, keepdim=True) + 1e-3).all()
 
 
+SHARES, ROW, STREAM_K, TILES, PAIRS = range(5)   # plan[0] of eet_gemm_w8a16_plan
+
+
+def _plan(M, N, K):
+    import ctypes
+    from eet_b200._lib import check, lib
+    plan = (ctypes.c_int * 5)()
+    check(lib.eet_gemm_w8a16_plan(M, N, K, plan))
+    return tuple(plan)
+
+
+@pytest.mark.parametrize("K,N,M,kernels", [
+    (4096, 32000, 384, (TILES, PAIRS)),    # stream-K 148 us, tiles 100, pairs 94
+    (8192, 22016, 384, (TILES, PAIRS)),    # 172, 134
+    (8192, 8192, 384, (TILES,)),           # 66, 50
+    (13696, 5120, 384, (TILES,)),          # 67, 55
+    (5120, 13696, 256, (TILES,)),          # 50, 39
+    (4096, 1536, 512, (STREAM_K,)),        # 17.2, 19.3
+    (4096, 4096, 100, (STREAM_K,))])       # 14.5, 17.5
+def test_models_choose_the_measured_kernel(K, N, M, kernels):
+    assert _plan(M, N, K)[0] in kernels
+
+
+def test_no_second_launch_of_more_clusters_of_three_than_find_room():
+    """8192 x 8192 at M = 1200 among others: 44 clusters of three behind a wave of single CTAs run in two turns."""
+    for K, N in ((8192, 8192), (8192, 24576), (4096, 12288), (4096, 4096)):
+        for M in range(300, 3100, 100):
+            kernel, _, whole, left, split = _plan(M, N, K)
+            assert not (kernel == TILES and whole > 0 and split == 3 and left > 40)
+
+
 @pytest.mark.parametrize("M", [1, 2, 3, 8, 9, 16])
 @pytest.mark.parametrize("KN", [(64, 64), (128, 192), (256, 64), (1024, 320)])
 def test_small_shapes(KN, M):
