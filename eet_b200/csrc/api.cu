@@ -286,8 +286,8 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
                                 route.pair.bn, (cudaStream_t)stream);
     }
     if (route.kernel == kRouteTiles) {
-        return launch_gemm_tc((const __half*)A, (const uint8_t*)packedB, (const __half*)scale, (__half*)C, res, gate, M, N,
-                              K, (cudaStream_t)stream);
+        return launch_gemm_tc((const __half*)A, (const uint8_t*)packedB, (const __half*)scale, (__half*)C, res, gate, M, N, K,
+                              route.tc, (cudaStream_t)stream);
     }
     // sums into the fp32 scratch, then one epilogue pass: all rows at once on the stream-K tensor-core kernel, in groups of
     // rows on the equal-share kernel

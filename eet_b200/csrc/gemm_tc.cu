@@ -737,6 +737,9 @@ static Tc2Plan tc2_plan(int M, int N, int K)
         const char* e = getenv("EET_TC2_SPLIT");
         forced = e ? atoi(e) : -1;
     }
+    // (looked up once: this runs before every launch)
+    int clusters[5];
+    for (int sp = 2; sp <= 4; ++sp) clusters[sp] = tc2_max_clusters(sp);
     Tc2Plan best = {0, 0, 0, 1, 1e30};
     for (int bn = M < 256 ? (M + 15) / 16 * 16 : 256; bn >= 32; bn -= 16) {
         const long long tiles_ll = (long long)tiles_n * ((M + bn - 1) / bn);
@@ -745,7 +748,7 @@ static Tc2Plan tc2_plan(int M, int N, int K)
         const double block = tc2_block_us(bn), epilogue = 1.5 + 0.01 * bn;
         for (int sp = 1; sp <= 4; ++sp) {
             const int left = sp > 1 ? tiles % G : 0, whole = tiles - left;
-            if (sp > 1 && (left == 0 || KT / sp < 4 || left > tc2_max_clusters(sp))) continue;
+            if (sp > 1 && (left == 0 || KT / sp < 4 || left > clusters[sp])) continue;
             if (forced >= 0 && sp != 1 && sp != forced) continue;
             // behind a wave of single CTAs the last few clusters of three find no room until others end and take a second turn
             // (8192 x 8192, M = 1200, 44 of them: 174 us; 12 clusters of four, BN = 256: 150)
@@ -784,7 +787,7 @@ Tc2Plan gemm_tc_plan(int M, int N, int K)
 }
 
 int launch_gemm_tc(const __half* A, const uint8_t* B, const __half* scale, __half* C, const __half* residual, int gate,
-                   int M, int N, int K, cudaStream_t stream)
+                   int M, int N, int K, const Tc2Plan& plan, cudaStream_t stream)
 {
     EET_CHECK(gemm_tc_supported(M, N, K), "tensor-core GEMM: needs M >= 65, N %% 128 == 0, K %% 64 == 0");
     EncodeTiledFn encode = encode_tiled_fn();
@@ -798,7 +801,6 @@ int launch_gemm_tc(const __half* A, const uint8_t* B, const __half* scale, __hal
         EET_CUDA(cudaFuncSetAttribute(gemm_tc2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_set[dev] = true;
     }
-    const Tc2Plan plan = tc2_plan(M, N, K);
     EET_CHECK(plan.bn > 0, "tensor-core GEMM: no plan for M=%d N=%d K=%d", M, N, K);
     CUtensorMap map;
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};

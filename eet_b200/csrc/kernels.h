@@ -57,7 +57,7 @@ struct Tc2Plan {
 };
 Tc2Plan gemm_tc_plan(int M, int N, int K);
 int launch_gemm_tc(const __half* A, const uint8_t* B, const __half* scale, __half* C, const __half* residual, int gate,
-                   int M, int N, int K, cudaStream_t stream);
+                   int M, int N, int K, const Tc2Plan& plan, cudaStream_t stream);
 
 // gemm_pair.cu (tcgen05 on CTA pairs)
 struct PairPlan {
