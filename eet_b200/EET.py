@@ -288,7 +288,7 @@ def gemm_w8a16(x, packed_w, scale, out=None, residual=None, gate=None):
         out = torch.empty((M, N), dtype=torch.float16, device=x.device)
     if gate is not None and residual is not None:
         raise RuntimeError("gemm_w8a16: residual and gate exclude each other")
-    if M <= _ROW_MAX_M and gate is None and (residual is None or residual.numel() > 0) and M > 0:
+    if 0 < M <= _ROW_MAX_M and N <= _ROW_MAX_N and gate is None and (residual is None or residual.numel() > 0):
         return _gemm_row(x, packed_w, scale, out, M, residual=residual)
     second, epilogue = (gate, 2) if gate is not None else (residual, 1 if residual is not None else 0)
     ws_bytes = lib.eet_gemm_w8a16_workspace_bytes(M, N, K)
@@ -298,7 +298,8 @@ def gemm_w8a16(x, packed_w, scale, out=None, residual=None, gate=None):
     return out
 
 
-_ROW_MAX_M = 16   # rows of the decode GEMM that finishes its product itself
+_ROW_MAX_M = 16      # rows of the decode GEMM that finishes its product itself
+_ROW_MAX_N = 16384   # wider matrices may be read faster by two launches with scratch: eet_gemm_w8a16 knows
 
 
 def _gemm_row(x, w, scale, out, M, w2=None, scale2=None, residual=None, norm=None, squares_out=None):

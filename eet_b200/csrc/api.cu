@@ -205,7 +205,7 @@ int eet_gemm_w8a16_finalize(float* sums, const void* scale, const void* residual
     return launch_finalize(sums, (const __half*)scale, (const __half*)residual, (__half*)C, M, N, (cudaStream_t)stream);
 }
 
-// Which kernel a shape goes to.  Up to 16 rows the row kernel.  Above that stream-K units into fp32 scratch with a finishing
+// Which kernel a shape goes to.  Up to 16 rows the row kernel, or equal shares with a finishing launch.  Above that stream-K units into fp32 scratch with a finishing
 // launch, tiles on single CTAs or tiles on CTA pairs, both with the epilogue fused: the shortest modelled time decides, among
 // those that the shape may take.  Measured on both sides of the lines: 4096 x 4096, M = 128 units 15 us, tiles 18, and at M = 256
 // 21.7 and 20.2; 4096 x 32000, M = 384 units 148, tiles 100, pairs 94; 11008 x 4096, M = 4096 single CTAs 267, pairs 249.
@@ -222,7 +222,7 @@ static GemmRoute gemm_route(int M, int N, int K)
 {
     GemmRoute r = {kRouteShares, true, Tc2Plan{0, 0, 0, 1, 1e30}, PairPlan{0, 1e30}};
     if (M <= kRowMaxM) {
-        r.kernel = kRouteRow;
+        if (!gemm_row_wastes_a_wave(M, N, K)) r.kernel = kRouteRow;
         return r;
     }
     const bool sums = M <= mid_use_max_m() && gemm_mid_supported(M, N, K) && !gemm_tc_owns(M, N, K);

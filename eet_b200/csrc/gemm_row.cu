@@ -6,7 +6,8 @@
 // memory for another launch to finish.  Here a CTA - or a cluster of 2 to 8 that splits the reduction - owns a whole
 // tile row (64 channels) and stores fp16.  Equal shares are not what HBM needs: it needs about 10 MB in flight, which
 // 150 CTAs with 64 KiB each give whatever the number of rows, so uneven rows per SM cost nothing until an SM has to
-// convert faster than it can (about 90 B/cycle against the 24 of its share of HBM).
+// convert faster than it can (about 90 B/cycle against the 24 of its share of HBM) - up to two rows per SM.  More rows run in
+// waves, and a last wave of few CTAs has too little in flight: see gemm_row_wastes_a_wave.
 //
 //  * Eight warps, each with a ring of its own (two 4 KiB tiles, filled by 1-D bulk copies that its lane 0 issues):
 //    warp w takes tiles w, w + 8, ... of the CTA's share of the row.  No producer warp, no barrier between warps until
@@ -352,15 +353,38 @@ int launch_row(const RowGemmArgs& a, cudaStream_t stream)
 
 }  // namespace
 
+// A wide matrix whose last wave of tile rows is mostly empty: the equal shares of gemm_skinny.cu read it faster, with a finishing
+// launch (3 us) and all, when what stays empty is worth more than 50 MB of weights.  M = 8: 8192 x 22016 (130 MB empty) 30.3 us
+// against 34.1 here, 8192 x 24576 (109) 33.3, 35.6; 5120 x 22016 (81) 20.5, 24.3; 4096 x 24576 (55) 18.8, 20.4; 4096 x 28672
+// (38) 21.3, 21.2; 4096 x 32000 (24) 23.7, 22.4.  Above 8 rows that kernel is bound by the activations (8192 x 22016 at M = 16
+// 39.1, 36.9) and the faster one only where the last wave is as good as empty (8192 x 19456, 304 rows: 33.9, 35.4).
+bool gemm_row_wastes_a_wave(int M, int N, int K)
+{
+    const int rows = N / kTile, slots = 2 * sm_count();
+    const int empty = rows > slots ? (rows + slots - 1) / slots * slots - rows : 0;
+    const double bytes = (double)empty * kTile * K;
+    return M <= 8 ? bytes > 50e6 : bytes > 100e6 && empty > 0.85 * rows;
+}
+
 int launch_gemm_row(RowGemmArgs a, cudaStream_t stream)
 {
     EET_CHECK(a.M <= kRowMaxM, "decode GEMM: M=%d exceeds %d", a.M, kRowMaxM);
     if (a.M == 0) return 0;
     // Two CTAs fit on an SM.  Fewer rows than SMs: as many CTAs per row as there is room for (4096 x 4096: four, 4.8 us),
-    // each with at least one tile per warp; a row per CTA otherwise (4096 x 12288: 192 CTAs, 9.1 us).
-    const int rows = a.N / kTile, room = 2 * sm_count() / rows;
+    // each with at least one tile per warp.  More, up to two per SM: a row per CTA (4096 x 12288: 192 CTAs, 9.1 us).  More
+    // than that run in waves; two CTAs per row where that leaves 70 MB less of the last wave empty (344 rows, 1.5 waves
+    // instead of 2: 8192 x 22016 at M = 16 36.9 us instead of 41.0, gate and up together at M = 8 60.5 instead of 66.5;
+    // 4096 x 22016, 39 MB: 22.2 instead of 20.5).
+    const int rows = a.N / kTile, slots = 2 * sm_count(), KT = a.K / kTile;
     int s = 1;
-    while (s < kRowMaxSplits && s + 1 <= room && (a.K / kTile) / (s + 1) >= kRowWarps) ++s;
+    if (rows > slots) {
+        const int half_waves = 2 * ((rows + slots - 1) / slots) - (2 * rows + slots - 1) / slots;   // saved by two CTAs per row
+        if ((double)half_waves * slots * kTile * a.K * (a.B2 != nullptr ? 2 : 1) / 2 > 70e6) s = 2;
+    }
+    else {
+        const int room = slots / rows;
+        while (s < kRowMaxSplits && s + 1 <= room && KT / (s + 1) >= kRowWarps) ++s;
+    }
     a.splits = s < 5 ? s : (s < 8 ? 4 : 8);
     const bool norm = a.gamma != nullptr;
     if (a.M <= 8) {

@@ -46,6 +46,7 @@ struct RowGemmArgs {
     int M, N, K, gate;
     int splits;              // CTAs per tile row, chosen by the launcher
 };
+bool gemm_row_wastes_a_wave(int M, int N, int K);   // the skinny kernel is the faster one
 int launch_gemm_row(RowGemmArgs a, cudaStream_t stream);
 
 // gemm_tc.cu (tcgen05 / TMEM)
