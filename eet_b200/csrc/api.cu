@@ -436,6 +436,15 @@ int eet_prefill_mha(const void* q, const void* kcache, const void* vcache, void*
                               T_max, pad_len, (const __half*)alibi, alibi_stride, (cudaStream_t)stream);
 }
 
+int eet_decode_mha_plan(int B, int H, int len, int* plan)
+{
+    EET_CHECK(B > 0 && H > 0 && len > 0 && plan != nullptr, "eet_decode_mha_plan: B, H and len must be positive and plan not NULL");
+    const AttnPlan p = attn_plan(B * H, len, 0);
+    plan[0] = p.splits;
+    plan[1] = p.ctas;
+    return 0;
+}
+
 int eet_decode_mha(const void* qkv, float* qkv_sums, const void* qkv_scale, void* kcache, void* vcache, void* ctx,
                    int B, int H, int D, int T_max, int step, const int* step_dev, const int64_t* pad_len,
                    const void* alibi, int alibi_stride, const float* alibi_slopes, int rope, float rope_base, int splits,

@@ -34,11 +34,9 @@ constexpr int kHalfWarps = kAttnConsumerThreads / 16;
 #ifndef EET_ATTN_TILE
 #define EET_ATTN_TILE 32
 #define EET_ATTN_STAGES 2
-#define EET_ATTN_CTAS 4
 #endif
 constexpr int kAttnTile = EET_ATTN_TILE;                     // time steps per shared-memory stage
 constexpr int kAttnStages = EET_ATTN_STAGES;
-constexpr int kAttnCtasPerSm = EET_ATTN_CTAS;
 constexpr int kAttnRowBytes = 256;                        // D = 128 halves
 constexpr int kAttnStageBytes = 2 * kAttnTile * kAttnRowBytes;  // K tile + V tile
 
@@ -104,12 +102,15 @@ struct AttnSmem {
 //
 // Data path: the history slice of a CTA is contiguous in the [B][H][T][D] caches, so a producer warp
 // streams it with 1-D bulk copies (TMA engine) of 32 time steps of K and of V per stage into a two-stage
-// ring; four CTAs per SM keep ~128 KiB in flight, and 96 registers a thread hold a tile's K and V pieces (with five CTAs the
-// 72 registers left spilled: the op at 8 x 1000 tokens 46.0 us, now 42.9; a decode step of 4 layers 269.8, now 259.9; three
-// CTAs leave room for no split of a history at 8 x 32 heads: 49.3 and 271.6).  Register-level loads of the same bytes stall
-// on the number of outstanding L1 misses long before HBM is busy.  Four consumer warps take a half-warp per time
-// step from shared memory.
-__global__ void __launch_bounds__(kAttnThreads, kAttnCtasPerSm)
+// ring; four or five CTAs per SM keep 128 or 160 KiB in flight.  Register-level loads of the same bytes stall on the number of
+// outstanding L1 misses long before HBM is busy.  Four consumer warps take a half-warp per time step from shared memory.
+//
+// kCtas is the number of CTAs per SM that the registers are dealt out for.  With four, 96 a thread hold a tile's K and V pieces;
+// with five the 72 left spill a little, which costs about 12 % (8 x 32 heads, 1000 steps: 27.0 us against 24.3) and is
+// worth it only where five need fewer waves or allow another split (launch_decode_mha).  Three leave no room for a split at
+// 8 x 32 heads (the op 49.3 us, against 42.9).
+template<int kCtas>
+__global__ void __launch_bounds__(kAttnThreads, kCtas)
 decode_mha_kernel(DecodeAttnArgs a)
 {
     constexpr int D = 128;
@@ -617,37 +618,58 @@ prefill_mha_kernel(const __half* __restrict__ q, const __half* __restrict__ kcac
 
 }  // namespace
 
+// CTAs per (batch, head) pair, and per SM, for `pairs` histories of up to `len` steps: with either number per SM as many CTAs as fit
+// on the machine at once, at least 64 steps each.  Four per SM are the faster code, so five are taken only where they leave
+// each CTA slot less to do: waves x 1 / splits.  Measured at 1000 steps, five against four: 5 x 32 heads (4 splits, 2)
+// 18.4 us against 20.2; 8 x 40 (2, 1) 33.3, 39.8; 18 x 40 at 500 (1 wave, 2) 34.9, 43.8; 32 x 40 at 500 (2 waves, 3) 58.7, 65.5;
+// equal: 8 x 32 27.0, 24.3; 10 x 40 51.2, 41.6; 24 x 40 at 500 53.6, 46.4.
+AttnPlan attn_plan(int pairs, int len, int splits)
+{
+    AttnPlan best = {1, 4};
+    double least = 1e30;
+    for (int ctas = 4; ctas <= 5; ++ctas) {
+        const int slots = ctas * sm_count();
+        int s = splits;
+        if (s == 0) {
+            const int room = slots / pairs;
+            s = 1;
+            while (s < 8 && s * 2 <= room && len / (s * 2) >= 64) s *= 2;
+            // more pairs than CTA slots: the launch runs in waves, and for long histories halves balance the last wave
+            // better (measured at 1024 pairs: +13 % at 1060 steps, -10 % at 320)
+            if (room == 0 && len >= 768) s = 2;
+        }
+        const double waves = (double)(((long long)pairs * s + slots - 1) / slots) / s;
+        if (waves < least) {
+            least = waves;
+            best = AttnPlan{s, ctas};
+        }
+    }
+    return best;
+}
+
 int launch_decode_mha(const DecodeAttnArgs& a, cudaStream_t stream)
 {
     EET_CHECK(a.D == 128, "decode attention: head size %d is not supported (128 only)", a.D);
     EET_CHECK(a.step_dev != nullptr || (a.step >= 1 && a.step <= a.T_max),
               "decode attention: step %d outside the cache length %d", a.step, a.T_max);
     if (a.B == 0) return 0;
-    int splits = a.splits;
-    if (splits == 0) {
-        // as many CTAs as fit on the machine at once (four per SM); at least 64 time steps per CTA
-        const int len = a.step_dev ? a.T_max : a.step;
-        const int room = kAttnCtasPerSm * sm_count() / (a.B * a.H);
-        splits = 1;
-        while (splits < 8 && splits * 2 <= room && len / (splits * 2) >= 64) splits *= 2;
-        // more (batch, head) pairs than CTA slots: the launch runs in waves, and for long histories halves
-        // balance the last wave better (measured at 1024 pairs: +13 % at 1060 steps, -10 % at 320)
-        if (room == 0 && len >= 768) splits = 2;
-    }
+    const AttnPlan plan = attn_plan(a.B * a.H, a.step_dev ? a.T_max : a.step, a.splits);
+    const int splits = plan.splits;
+    auto kern = plan.ctas == 5 ? decode_mha_kernel<5> : decode_mha_kernel<4>;
     EET_CHECK(splits == 1 || splits == 2 || splits == 4 || splits == 8, "decode attention: splits must be 1,2,4,8");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(splits, a.B * a.H, 1);
     cfg.blockDim = dim3(kAttnThreads, 1, 1);
     cfg.dynamicSmemBytes = kAttnStages * kAttnStageBytes;
     if (kAttnStages * kAttnStageBytes > 48 * 1024) {
-        static bool attr_set[64] = {};
+        static bool attr_set[64][2] = {};
         int dev = 0;
         EET_CUDA(cudaGetDevice(&dev));
         dev &= 63;
-        if (!attr_set[dev]) {
-            EET_CUDA(cudaFuncSetAttribute(decode_mha_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (!attr_set[dev][plan.ctas == 5]) {
+            EET_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           kAttnStages * kAttnStageBytes));
-            attr_set[dev] = true;
+            attr_set[dev][plan.ctas == 5] = true;
         }
     }
     cfg.stream = stream;
@@ -660,7 +682,7 @@ int launch_decode_mha(const DecodeAttnArgs& a, cudaStream_t stream)
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    EET_CUDA(cudaLaunchKernelEx(&cfg, decode_mha_kernel, a));
+    EET_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
     return 0;
 }
 

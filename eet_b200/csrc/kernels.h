@@ -122,6 +122,10 @@ struct DecodeAttnArgs {
     float rope_base;
     int splits;               // CTAs per (batch, head): 1, 2, 4 or 8; 0 = choose
 };
+struct AttnPlan {
+    int splits, ctas;   // CTAs per (batch, head) pair, CTAs per SM
+};
+AttnPlan attn_plan(int pairs, int len, int splits);
 int launch_decode_mha(const DecodeAttnArgs& a, cudaStream_t stream);
 int launch_prefill_mha(const __half* q, const __half* kcache, const __half* vcache, __half* ctx, int B, int S, int H,
                        int D, int T_max, const int64_t* pad_len, const __half* alibi, int alibi_stride,

@@ -262,6 +262,10 @@ int eet_decode_mha(const void* qkv, float* qkv_sums, const void* qkv_scale, void
                    const void* alibi, int alibi_stride, const float* alibi_slopes, int rope, float rope_base, int splits,
                    void* stream);
 
+/* What splits = 0 chooses on the current device for histories of up to `len` steps, for tests and tools; launches nothing:
+ * plan[0] CTAs per (batch, head), plan[1] CTAs per SM that the kernel is built for (4 or 5). */
+int eet_decode_mha_plan(int B, int H, int len, int* plan);
+
 /* Scratch needed by eet_reorder_kv: 2 * B * H * step * D halves. */
 size_t eet_reorder_kv_workspace_bytes(int B, int H, int D, int step);
 

@@ -61,6 +61,37 @@ def test_decode_rope(step, splits):
     assert torch.equal(kc_host, kh)
 
 
+def _decode_plan(B, H, length):
+    import ctypes
+    from eet_b200._lib import check, lib
+    plan = (ctypes.c_int * 2)()
+    check(lib.eet_decode_mha_plan(B, H, length, plan))
+    return tuple(plan)
+
+
+@pytest.mark.parametrize("B,H,length,plan", [
+    # us with five CTAs per SM, and with four as its rule would split
+    (8, 40, 1000, (2, 5)), (5, 32, 1000, (4, 5)), (18, 40, 500, (1, 5)), (32, 40, 500, (1, 5)),   # 33 / 40, 18 / 20, 35 / 44, 59 / 66
+    (8, 32, 1000, (2, 4)), (10, 40, 1000, (1, 4)), (24, 40, 500, (1, 4)), (1, 32, 1000, (8, 4))])  # 27 / 24, 51 / 42, 54 / 46, 9.0 / 7.5
+def test_decode_takes_five_ctas_per_sm_where_they_save_a_wave_or_a_split(B, H, length, plan):
+    assert _decode_plan(B, H, length) == plan
+
+
+@pytest.mark.parametrize("B,H,step", [(8, 40, 140), (16, 40, 33), (5, 32, 270)])
+def test_decode_with_five_ctas_per_sm(B, H, step):
+    D, T = 128, step + 3
+    assert _decode_plan(B, H, step)[1] == 5
+    gen = torch.Generator().manual_seed(step)
+    qkv = torch.randn(B, 3, H, D, generator=gen).half()
+    kh = torch.randn(B, H, T, D, generator=gen).half()
+    vh = torch.randn(B, H, T, D, generator=gen).half()
+    pad = torch.arange(B, dtype=torch.long) % step
+    ref, _, vc_ref = _oracle_decode(qkv, kh, vh, step, pad, None, True)
+    kc, vc = kh.cuda(), vh.cuda()
+    assert _close(_decode(qkv.cuda(), kc, vc, step, pad=pad.view(B, 1).cuda()), ref)
+    assert torch.equal(vc.cpu(), vc_ref)
+
+
 def test_decode_beyond_the_reference_4096_limit():
     B, H, D, T, step = 1, 2, 128, 5000, 4800
     gen = torch.Generator().manual_seed(1)
