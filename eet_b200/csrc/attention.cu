@@ -95,6 +95,7 @@ struct AttnSmem {
     // copy of this structure through distributed shared memory
     float c_acc[8][128];
     float c_ml[8][2];
+    uint32_t sink[kAttnConsumerWarps];   // see reads_returned
     volatile int abort;
 };
 
@@ -271,6 +272,7 @@ decode_mha_kernel(DecodeAttnArgs a)
             const uint4* vt = kt + kAttnTile * (kAttnRowBytes / 16);
             const int t0 = t_first + j * kAttnTile;
             uint4 kv[U], vv[U];
+            uint32_t words = 0;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int r = hw + u * kHalfWarps;
@@ -283,8 +285,10 @@ decode_mha_kernel(DecodeAttnArgs a)
                     kv[u] = kt[r * (kAttnRowBytes / 16) + hl];
                     vv[u] = vt[r * (kAttnRowBytes / 16) + hl];
                 }
+                words ^= kv[u].x ^ vv[u].x;
             }
             // the tile's bytes are in registers: hand the stage back to the producer
+            reads_returned(words, &sm.sink[warp]);
             __syncwarp();
             if ((tid & 31) == 0) mbar_arrive(&sm.empty[s]);
             // the U time steps of this half-warp are folded into the running softmax together: independent

@@ -115,6 +115,17 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     return false;
 }
 
+// Before a warp hands a shared-memory stage back to the copy engine, its reads of the stage must have returned.  An mbarrier
+// arrival does not wait for them: reads held up behind another kernel's memory traffic on the same SM (under programmatic
+// dependent launch the preceding kernel's last CTAs) were passed by the arrival and saw the next copy's bytes, in 1 of 100
+// calls of the stream-K GEMM behind a finishing launch.  Instructions issue in order, and a store that needs a word of every
+// read cannot issue before they have returned, so the arrival behind it cannot either.  `words`: one word of each read,
+// combined; `sink`: a word that nobody reads.
+__device__ __forceinline__ void reads_returned(uint32_t words, uint32_t* sink)
+{
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_u32(sink)), "r"(words) : "memory");
+}
+
 // 1-D bulk copy global -> shared through the TMA engine; completion is signalled on `bar` as
 // transaction bytes.  Both addresses must be 16-byte aligned and `bytes` a multiple of 16.
 __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar)

@@ -67,6 +67,7 @@ struct MidSmem {
     uint64_t h_ready[kMidNHMax], h_empty[kMidNHMax];    // fp16 weights written (4 warps) / their MMAs completed
     uint64_t acc_full[2];                               // all MMAs of a strip segment have completed
     uint64_t acc_empty[2];                              // the epilogue warps have read the accumulator buffer (4 warps)
+    uint32_t sink[4];                                   // see reads_returned
     uint32_t tmem_base;
     volatile int abort;
 };
@@ -297,16 +298,19 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, GemmArgs a)
             const int nk = (kp * kMidUnitK + 1 < KT) ? 2 : 1;
             const uint8_t* row = w_ring + (size_t)sw * kMidWStage + row_off;
             uint4 c[kMidUnitK][4];
+            uint32_t words = 0;
 #pragma unroll
             for (int kk = 0; kk < kMidUnitK; ++kk) {
                 if (kk < nk) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         c[kk][j] = *reinterpret_cast<const uint4*>(row + kk * kTileBytes + ((j ^ sxr) << 4));
+                        words ^= c[kk][j].x;
                     }
                 }
             }
             // the int8 stage is free again as soon as the bytes are in registers
+            reads_returned(words, &sm.sink[warp & 3]);
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.w_empty[sw]);
             bool live = true;

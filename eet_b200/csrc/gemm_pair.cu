@@ -267,8 +267,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __re
                         cvt_u8x4_to_f16x4(raw.w, o[pass][1].z, o[pass][1].w);
                     }
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sm.w_empty[sw]);
                 if (it >= kPrNH) {
                     if (!tc_wait_warp(&sm.done[d], phd, &sm.abort)) {
                         ok = false;
@@ -291,7 +289,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __re
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(ready[sh]);
+                // (the int8 stage goes back only now: the stores above could not issue before their reads of it had returned)
+                if (lane == 0) {
+                    mbar_arrive_cluster(ready[sh]);
+                    mbar_arrive(&sm.w_empty[sw]);
+                }
                 if (++sw == kPrNW) {
                     sw = 0;
                     phw ^= 1;

@@ -64,6 +64,7 @@ gemm_row_kernel(RowGemmArgs a)
 {
     extern __shared__ __align__(128) uint8_t row_dyn[];   // [warp][slot] tiles | partial sums of the other ranks
     __shared__ uint64_t full[kRowWarps][kRowSlots];
+    __shared__ uint32_t sink[kRowWarps];                  // see reads_returned
     pdl_launch_dependents();
     constexpr int kMats = kPair ? 2 : 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -187,12 +188,14 @@ gemm_row_kernel(RowGemmArgs a)
                 g_device_status = 1;
             }
             const uint8_t* w = ring + slot * kTileBytes + lane * 16;
+            uint32_t words = 0;
 #pragma unroll
             for (int cg = 0; cg < 4; ++cg) {
                 const uint4 wa = *reinterpret_cast<const uint4*>(w + cg * 1024);
                 const uint4 wb = *reinterpret_cast<const uint4*>(w + cg * 1024 + 512);
                 const uint32_t wa4[4] = {wa.x, wa.y, wa.z, wa.w};
                 const uint32_t wb4[4] = {wb.x, wb.y, wb.z, wb.w};
+                words = wb.w;   // (a warp's reads return in order)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     uint32_t a0, a1, a2, a3;
@@ -204,6 +207,7 @@ gemm_row_kernel(RowGemmArgs a)
                     }
                 }
             }
+            reads_returned(words, &sink[warp]);
             __syncwarp();
             const int q = kMats * j + p + kRowSlots;
             if (lane == 0 && live && q < kMats * mine) issue(q, slot);

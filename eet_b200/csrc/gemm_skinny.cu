@@ -67,6 +67,7 @@ struct SkinnySmem {
     uint64_t full[kMaxStages];
     uint64_t empty[kMaxStages];
     float fold[4][2][32][4];  // fragments of warps 4-7 on their way to warps 0-3 at the end of a tile row
+    uint32_t sink[kConsumerWarps];   // see reads_returned
     volatile int abort;
 };
 
@@ -231,6 +232,7 @@ gemm_skinny_kernel(GemmArgs a)
         const uint8_t* stage = dyn_smem + (size_t)s * kStageBytes;
         const uint8_t* ws = stage + cg * 1024 + lane * 16;
         const uint8_t* xs = stage + kStageWBytes + tq * 32;
+        uint32_t words = 0;
 #pragma unroll
         for (int t = 0; t < kStageTiles / 2; ++t) {
             const int tile = kh * (kStageTiles / 2) + t;
@@ -248,6 +250,7 @@ gemm_skinny_kernel(GemmArgs a)
                 }
                 const uint4 wa = *reinterpret_cast<const uint4*>(ws + tile * kTileBytes);
                 const uint4 wb = *reinterpret_cast<const uint4*>(ws + tile * kTileBytes + 512);
+                words = wb.w;   // (a warp's reads return in order)
                 const uint32_t wa4[4] = {wa.x, wa.y, wa.z, wa.w};
                 const uint32_t wb4[4] = {wb.x, wb.y, wb.z, wb.w};
 #pragma unroll
@@ -262,6 +265,7 @@ gemm_skinny_kernel(GemmArgs a)
                 }
             }
         }
+        reads_returned(words, &sm.sink[warp]);
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.empty[s]);
         g += nb_tiles;

@@ -497,8 +497,6 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
                         cvt_u8x4_to_f16x4(raw.w, o[pass][1].z, o[pass][1].w);
                     }
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sm.w_empty[sw]);
                 if (it >= kTc2NH) {
                     if (!tc_wait_warp(&sm.done[d], phd, &sm.abort)) {
                         ok = false;
@@ -521,8 +519,10 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
+                // (the int8 stage goes back only now: the stores above could not issue before their reads of it had returned)
                 if (lane == 0) {
                     mbar_arrive(&sm.h_ready[sh]);
+                    mbar_arrive(&sm.w_empty[sw]);
                 }
                 if (++sw == nw) {
                     sw = 0;

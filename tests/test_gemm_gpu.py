@@ -84,6 +84,27 @@ def test_wide_matrices_of_few_rows_avoid_an_empty_wave(K, N, M, kernel):
         assert torch.equal(EET.gemm_w8a16(x, packed, s, residual=r), out)
 
 
+@pytest.mark.parametrize("K,N,M", [(4096, 4096, 128), (4096, 4096, 250), (4096, 4096, 40), (4096, 11008, 17), (4096, 12288, 300),
+                                   (4096, 4096, 1200), (4096, 4096, 8), (4096, 12288, 16), (4096, 22016, 8), (4096, 192, 100)])
+def test_calls_behind_one_another_give_the_same_bits(K, N, M):
+    """Six hundred calls that nothing waits between, each kernel beginning beside the last CTAs of the one before it: reads of
+    a weight stage that are held up by that kernel's memory traffic must not see the stage's next bytes.  Small whole numbers
+    as activations, so every fp32 sum is exact whatever the order of the additions."""
+    from eet_b200 import EET, _lib
+    gen = torch.Generator(device="cuda").manual_seed(N + M)
+    q = torch.randint(-127, 128, (K, N), generator=gen, device="cuda", dtype=torch.int8)
+    s = torch.full((N,), 2.0 ** -10, device="cuda").half()
+    x = torch.randint(-4, 5, (M, K), generator=gen, device="cuda").half()
+    packed = EET.preprocess_weights(q)
+    want = ((x.double() @ q.double()) * 2.0 ** -10).half()
+    outs = torch.empty(50, M, N, dtype=torch.float16, device="cuda")
+    for _ in range(12):
+        for out in outs:
+            EET.gemm_w8a16(x, packed, s, out=out)
+        assert bool((outs == want).all())
+    assert _lib.device_status() == 0
+
+
 def test_no_second_launch_of_more_clusters_of_three_than_find_room():
     """8192 x 8192 at M = 1200 among others: 44 clusters of three behind a wave of single CTAs run in two turns."""
     for K, N in ((8192, 8192), (8192, 24576), (4096, 12288), (4096, 4096)):
