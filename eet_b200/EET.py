@@ -284,11 +284,12 @@ def gemm_w8a16(x, packed_w, scale, out=None, residual=None, gate=None):
     ops call it (csrc/op/llama_mmha.cpp:319-331)."""
     K, N = packed_w.shape
     M = x.numel() // K
+    in_place = out is not None and out.data_ptr() < x.data_ptr() + 2 * M * K and x.data_ptr() < out.data_ptr() + 2 * M * N
     if out is None:
         out = torch.empty((M, N), dtype=torch.float16, device=x.device)
     if gate is not None and residual is not None:
         raise RuntimeError("gemm_w8a16: residual and gate exclude each other")
-    if 0 < M <= _ROW_MAX_M and N <= _ROW_MAX_N and gate is None and (residual is None or residual.numel() > 0):
+    if 0 < M <= _ROW_MAX_M and N <= _ROW_MAX_N and not in_place and gate is None and (residual is None or residual.numel() > 0):
         return _gemm_row(x, packed_w, scale, out, M, residual=residual)
     second, epilogue = (gate, 2) if gate is not None else (residual, 1 if residual is not None else 0)
     ws_bytes = lib.eet_gemm_w8a16_workspace_bytes(M, N, K)

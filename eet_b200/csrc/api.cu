@@ -263,10 +263,13 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
               "eet_gemm_w8a16: epilogues 1 and 2 need a 16-byte aligned second operand");
     const __half* res = epilogue != 0 ? (const __half*)residual : nullptr;
     const int gate = epilogue == 2 ? 1 : 0;
-    const GemmRoute route = gemm_route(M, N, K);
+    GemmRoute route = gemm_route(M, N, K);
     EET_CHECK(!route.scratch || (ws && aligned16(ws) && ws_bytes >= eet_gemm_w8a16_workspace_bytes(M, N, K)),
               "eet_gemm_w8a16: workspace of %zu bytes is smaller than the %zu needed", ws_bytes,
               eet_gemm_w8a16_workspace_bytes(M, N, K));
+    // C over A: only sums that are finished by another launch let all of A be read before C is stored
+    const uintptr_t a0 = (uintptr_t)A, a1 = a0 + (size_t)M * K * 2, c0 = (uintptr_t)C, c1 = c0 + (size_t)M * N * 2;
+    if (route.scratch && a0 < c1 && c0 < a1) route.kernel = gemm_mid_supported(M, N, K) ? kRouteStreamK : kRouteShares;
     if (route.kernel == kRouteRow) {
         // decode regime: one launch that leaves the scratch alone (this entry point has always asked for it)
         RowGemmArgs r = {};

@@ -106,7 +106,8 @@ size_t eet_gemm_w8a16_workspace_bytes(int M, int N, int K);
  *             holds the gate projection: the reference's gated_act kernel (csrc/core/activation_kernel.cu:106-124,
  *             called from csrc/op/gated_ffn_int8.cpp:290-301) fused in, with its mix of fp32 and fp16 arithmetic.
  *   residual  device fp16 [M][N] for epilogues 1 and 2, else NULL (may alias C)
- * M may be any value >= 0; K and N must be multiples of 64; pointers 16-byte aligned.
+ * M may be any value >= 0; K and N must be multiples of 64; pointers 16-byte aligned.  C may lie over A up to 64 rows, and up
+ * to 512 for shapes that need the scratch.
  * Kernels: M <= 16 TMA-staged row kernel (one launch, leaves the scratch alone); 16 < M <= 512 (N % 128 == 0) stream-K tcgen05 kernel; above
  * that - and from M = 65 on for shapes (N % 256 == 0) whose 256 x 256 tiles, whole or with their k-blocks split
  * over clusters of 2-4 CTAs, can occupy most of the GPU - tcgen05 kernels with 256 x 256 or 128 x 256 output

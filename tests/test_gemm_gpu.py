@@ -105,6 +105,26 @@ def test_calls_behind_one_another_give_the_same_bits(K, N, M):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("epilogue", ["plain", "residual"])
+@pytest.mark.parametrize("n,M", [(4096, 3), (4096, 16), (1024, 8), (192, 9), (4096, 40), (4096, 100), (4096, 200), (192, 300)])
+def test_output_over_the_activations(n, M, epilogue):
+    """out=x: no value of x may be overwritten before every CTA has read it.  Repeated, on a busy queue."""
+    from eet_b200 import EET
+    gen = torch.Generator(device="cuda").manual_seed(n + M)
+    q = torch.randint(-127, 128, (n, n), generator=gen, device="cuda", dtype=torch.int8)
+    s = ((torch.rand(n, generator=gen, device="cuda") + 0.5) * n ** -0.5 / 64).half()
+    x = torch.randn(M, n, generator=gen, device="cuda").half()
+    r = torch.randn(M, n, generator=gen, device="cuda").half()
+    packed = EET.preprocess_weights(q)
+    y = (x.double() @ q.double()) * s.double()
+    want = y + (r.double() if epilogue == "residual" else 0)
+    bufs = [x.clone() for _ in range(20)]
+    for b in bufs:
+        EET.gemm_w8a16(b, packed, s, out=b, residual=r if epilogue == "residual" else None)
+    tol = 2.0 ** -10 * (y.abs() + want.abs()) + 1e-4
+    assert all(bool(((b.double() - want).abs() <= tol).all()) for b in bufs)
+
+
 def test_no_second_launch_of_more_clusters_of_three_than_find_room():
     """8192 x 8192 at M = 1200 among others: 44 clusters of three behind a wave of single CTAs run in two turns."""
     for K, N in ((8192, 8192), (8192, 24576), (4096, 12288), (4096, 4096)):
