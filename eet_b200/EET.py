@@ -91,7 +91,8 @@ class _Pool:
         key = (name, str(device), dtype)
         buf = self.buffers.get(key)
         if buf is None or buf.numel() < numel:
-            buf = torch.empty(max(int(numel), 1), dtype=dtype, device=device)
+            with torch.inference_mode(False):   # (its views count their changes, see _Squares; inference tensors don't)
+                buf = torch.empty(max(int(numel), 1), dtype=dtype, device=device)
             self.buffers[key] = buf
             self.views.clear()   # views of the buffer it replaces
         return buf
@@ -148,6 +149,8 @@ _pool = _Pool()
 
 def clear_buffers():
     """Drops the pooled scratch buffers (MManager::clear, csrc/op/mmanager.hpp:211-214)."""
+    for ptr in [k for k, p in _pending.items() if isinstance(p, _Squares)]:
+        del _pending[ptr]
     _pool.clear()
 
 
@@ -376,14 +379,16 @@ class _Pending:
 
 class _Squares:
     """Sums of squares of the 64-channel pieces of an op's (finished) output: the next op of this module that receives
-    the tensor normalises it while its first projection loads it."""
-    __slots__ = ("squares",)
+    the tensor normalises it while its first projection loads it.  They hold for `out` (kept, so that its address means
+    nothing else meanwhile) as long as nothing changes it: torch counts the changes of a tensor's memory that it makes."""
+    __slots__ = ("squares", "out", "shape", "version")
 
-    def __init__(self, squares):
-        self.squares = squares
+    def __init__(self, squares, out):
+        self.squares, self.out, self.shape, self.version = squares, out, out.shape, out._version
 
 
 _pending = {}
+_squares_at = {}   # cache name -> address of the output whose sums of squares its buffer holds
 _defer = [False]
 _DECODE_MAX_M = 64       # below the tensor-core GEMM's first M
 _DECODE_MAX_M_TP = 64    # rows of the tensor-parallel peer buffers (tp.PeerBuffers.ROWS)
@@ -401,15 +406,21 @@ def _project_row(x, w, scale, out, residual, M, desc, name):
     N = w.shape[1]
     squares = _pool.get("squares:" + name, _ROW_MAX_M * (N // 64), torch.float32, desc.device)
     _gemm_row(x, w, scale, out, M, residual=residual, squares_out=squares)
-    _pending[out.data_ptr()] = _Squares(squares)
+    ptr = out.data_ptr()
+    before = _squares_at.get(name)
+    if before is not None and before != ptr and isinstance(_pending.get(before), _Squares):
+        del _pending[before]   # an output in a buffer since replaced: its sums have just been written over
+    _squares_at[name] = ptr
+    _pending[ptr] = _Squares(squares, out)
 
 
 def _take_squares(x2d, gamma, desc):
     """The `norm` argument of _gemm_row for an input that such a chain has produced, else None."""
-    p = _pending.get(x2d.data_ptr())
-    if not isinstance(p, _Squares) or not _row_chain(x2d.shape[0], desc):
+    ptr = x2d.data_ptr()
+    p = _pending.get(ptr)
+    if not isinstance(p, _Squares) or x2d.shape != p.shape or p.version != p.out._version or not _row_chain(p.shape[0], desc):
         return None
-    del _pending[x2d.data_ptr()]
+    del _pending[ptr]
     return gamma, p.squares, desc.layernorm_eps
 
 
@@ -424,10 +435,13 @@ def _defer_ok(M, desc):
 
 
 class deferred_epilogue:
-    """Context manager for a chain of decode-step ops of this module (M <= 64): inside
-    it an attention / FFN op returns its output tensor *before* the last GEMM's epilogue has run, and the next
-    op (attention, FFN or LayerNorm of this module) completes it in its RMSNorm kernel.  Outputs still
-    unfinished when the context ends are completed then, so callers outside never see stale memory."""
+    """Context manager for a chain of decode-step ops of this module (M <= 64), each handed the output of the one before.
+    With more than 16 rows, or with tensor parallelism, an attention / FFN op inside it returns its output tensor *before*
+    the last GEMM's epilogue has run, and the next op (attention, FFN or LayerNorm of this module) completes it in its
+    RMSNorm kernel: nothing else may read or change it.  Outputs still unfinished when the context ends are completed
+    then, so callers outside never see stale memory.  Up to 16 rows on one GPU the output is finished, and its sums of
+    squares wait for the next op's norm; an output that torch changes in place is normalised afresh, one that something
+    else writes to (a kernel given its address) must not be handed on inside the context."""
 
     def __enter__(self):
         self.prev = _defer[0]

@@ -148,3 +148,40 @@ def test_pool_rows_follow_a_replaced_buffer():
     assert c.data_ptr() == b.data_ptr() != a.data_ptr()
     pool.clear()
     assert pool.rows("x", 2, 8, 32, torch.float16, dev).data_ptr() != 0 and not pool.gemm_ws
+
+
+def test_sums_of_squares_hold_for_the_unchanged_output_only(monkeypatch):
+    """What a decode projection leaves for the next op's norm: not for a tensor that was changed in place (also in
+    inference mode), not for another one, not once a later output's sums stand in the same buffer, not after
+    clear_buffers()."""
+    import types
+    monkeypatch.setattr(EET, "_gemm_row", lambda *a, **k: None)
+    desc = types.SimpleNamespace(is_int8=True, tp=None, layernorm_eps=1e-6, device=torch.device("cpu"))
+    w, gamma = torch.empty(64, 128), torch.ones(128)
+
+    def project(rows=2, capacity=4 * 128):
+        out = EET._pool.rows("cpu_test", rows, 128, capacity, torch.float16, desc.device)
+        EET._project_row(None, w, None, out, None, rows, desc, "cpu_test")
+        return out.view(1, rows, 128)
+    with EET.deferred_epilogue():
+        out = project()
+        assert EET._take_squares(out.view(2, 128), gamma, desc)[1].numel() >= 2 * 2
+        assert EET._take_squares(out.view(2, 128), gamma, desc) is None          # taken once
+        out = project()
+        assert EET._take_squares(out.view(2, 128)[:1], gamma, desc) is None      # other rows
+        out = project()
+        out.add_(1)
+        assert EET._take_squares(out.view(2, 128), gamma, desc) is None
+        with torch.inference_mode():
+            out = project(rows=3)
+            out.mul_(2)
+            assert EET._take_squares(out.view(3, 128), gamma, desc) is None
+        first = project()
+        second = project(rows=8, capacity=8 * 128)                               # a larger buffer, the same sums
+        assert first.data_ptr() != second.data_ptr()
+        assert EET._take_squares(first.view(2, 128), gamma, desc) is None
+        assert EET._take_squares(second.view(8, 128), gamma, desc) is not None
+        out = project()
+        EET.clear_buffers()
+        assert EET._take_squares(out.view(2, 128), gamma, desc) is None
+    assert not EET._pending

@@ -213,6 +213,38 @@ def test_decode_batch_above_16_uses_the_stream_k_kernel_and_matches_oracle():
     assert _lib.device_status() == 0
 
 
+def test_hidden_state_changed_in_place_between_two_ops_of_a_decode_step():
+    """A steering delta added to the attention op's output inside the deferred context: the FFN op normalises the changed
+    tensor, not with the sums of squares of the old one - the same bits as two ops on their own."""
+    from eet_b200 import EET
+    B, h, f, none = 8, 256, 512, torch.empty(0)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    desc = EET.MetaDesc(torch.float16, B, 2, h, 1, 8, 16, "silu", 128, f, "cuda:0", False, 1e-6, True)
+
+    def weight(K, N):
+        q = torch.randint(-127, 128, (K, N), generator=gen, device="cuda", dtype=torch.int8)
+        return EET.preprocess_weights(q), torch.full((N,), K ** -0.5 / 64, device="cuda").half()
+    ones = torch.ones(h, device="cuda").half()
+    (qkv, out), (gate, up, down) = (weight(h, 3 * h), weight(h, h)), (weight(h, f), weight(h, f), weight(f, h))
+    att = EET.LlamaMmha(desc, *qkv, none, none, none, *out, none, ones, none)
+    ffn = EET.GatedFeedForwardNetworkInt8(desc, *gate, none, *up, none, *down, none, ones, none)
+    att.forward(torch.randn(B, 4, h, generator=gen, device="cuda").half(), none, none, True, True, True, none)
+    x = torch.randn(B, 1, h, generator=gen, device="cuda").half()
+    delta = 5 * torch.randn(B, 1, h, generator=gen, device="cuda").half()
+
+    def step(change):
+        att.step_ = 4
+        y = att.forward(x, none, none, True, True, False, none)
+        if change:
+            y.add_(delta)
+        return ffn.forward(y, True, True).clone()
+    want, plain = step(True), step(False)
+    with EET.deferred_epilogue():
+        got, kept = step(True), step(False)
+    assert torch.equal(got, want)
+    assert torch.allclose(kept.float(), plain.float(), atol=2e-2, rtol=1e-2) and not torch.allclose(kept.float(), want.float(), atol=0.5)
+
+
 def test_int8_lm_head_logits_and_greedy_choice():
     """lm_head_int8=True (an option beyond the reference): the head is quantized like the other projections; its
     logits against the oracle with the same quantized head, and the fused greedy kernel against argmax of them."""
