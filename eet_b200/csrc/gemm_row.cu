@@ -134,8 +134,8 @@ gemm_row_kernel(RowGemmArgs a)
             xr[nb][0] = xr[nb][1] = make_uint4(0u, 0u, 0u, 0u);
             if (j < mine && gq + 8 * nb < a.M) {
                 const uint4* p = reinterpret_cast<const uint4*>(a.A + (size_t)(gq + 8 * nb) * a.K + (size_t)(t0 + i) * kTile + tq * 16);
-                xr[nb][0] = __ldg(p);
-                xr[nb][1] = __ldg(p + 1);
+                xr[nb][0] = p[0];   // (not __ldg: the preceding kernel writes them during this one's lifetime)
+                xr[nb][1] = p[1];
             }
         }
     };

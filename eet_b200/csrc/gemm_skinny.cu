@@ -181,8 +181,9 @@ gemm_skinny_kernel(GemmArgs a)
             const int tile = kh * kHalfTiles + (col >> 3);
             xr[u] = make_uint4(0, 0, 0, 0);
             if (c < kXChunks && row < rows && tile < nb_tiles_stage) {
-                xr[u] = __ldg(reinterpret_cast<const uint4*>(a.A + (size_t)(m0 + row) * a.K +
-                                                             (size_t)(kb_stage + kh * kHalfTiles) * kTile) + col);
+                // (not __ldg: the preceding kernel writes them during this one's lifetime)
+                xr[u] = reinterpret_cast<const uint4*>(a.A + (size_t)(m0 + row) * a.K +
+                                                       (size_t)(kb_stage + kh * kHalfTiles) * kTile)[col];
             }
         }
     };

@@ -30,3 +30,11 @@ def test_warps_whose_wait_ran_out_join_the_barrier_of_the_epilogue(name):
     assert not re.search(r"\b(break|return|continue|goto)\b", role[body_end:at])
     waits = re.findall(r"\btc_wait\w*\(", role[start:at])
     assert len(waits) == 3 and set(waits) == {"tc_wait_warp("}
+
+
+@pytest.mark.parametrize("name", ["gemm_row.cu", "gemm_skinny.cu"])
+def test_what_the_preceding_kernel_writes_is_not_read_as_constant(name):
+    """These kernels begin before the one in front of them has ended.  __ldg promises that nobody writes the memory during the
+    kernel's lifetime: true of weights, scales and norm weights, not of what is read behind pdl_wait."""
+    text = _source(name)
+    assert "__ldg" not in text[text.index("pdl_wait();"):]
