@@ -137,6 +137,7 @@ decode_mha_kernel(DecodeAttnArgs a)
     }
 
     pdl_launch_dependents();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // waited for before the first remote store
     __syncthreads();  // barriers initialised (before the wait below, so that nothing stands between it and the
                       // producer's first request)
     // everything this kernel reads that an earlier kernel of the same step produced (the projection of the
@@ -187,6 +188,8 @@ decode_mha_kernel(DecodeAttnArgs a)
                          (uint32_t)(rows * kAttnRowBytes), &sm.full[s]);
             }
         }
+        __syncwarp();
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     }
     else {
         // ---- new token: rotate q,k at position step-1, round to fp16 as the reference's buffers do ----
@@ -343,6 +346,7 @@ decode_mha_kernel(DecodeAttnArgs a)
             }
         }
 
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // every CTA of the cluster runs: rank 0's memory may be written
         // ---- merge the half-warps of this CTA ----
         if (hl == 0) {
             sm.m[hw] = st.m;

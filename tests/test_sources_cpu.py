@@ -38,3 +38,12 @@ def test_what_the_preceding_kernel_writes_is_not_read_as_constant(name):
     kernel's lifetime: true of weights, scales and norm weights, not of what is read behind pdl_wait."""
     text = _source(name)
     assert "__ldg" not in text[text.index("pdl_wait();"):]
+
+
+@pytest.mark.parametrize("name,push", [("attention.cu", "map_shared_rank("), ("gemm_row.cu", "st.shared::cluster"),
+                                       ("gemm_tc.cu", "st.shared::cluster")])
+def test_no_store_into_another_cta_before_it_is_known_to_run(name, push):
+    """A CTA may write another's shared memory only once that one has begun: a cluster barrier comes first."""
+    text = _source(name)
+    before = text[:text.index(push)]
+    assert "barrier.cluster.wait" in before or "this_cluster().sync()" in before
