@@ -29,7 +29,7 @@ ROOT = os.path.dirname(os.path.dirname(HERE))
 sys.path.insert(0, ROOT)
 from oracle import w8  # noqa: E402
 
-REF = os.environ.get("EET_REFERENCE", "/root/reference")
+REF = os.environ.get("EET_REFERENCE") or sys.exit("set EET_REFERENCE to a checkout of the reference")
 
 
 def quant_case(name, w):
