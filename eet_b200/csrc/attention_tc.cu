@@ -110,8 +110,9 @@ __device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint3
 
 // The ALiBi bias of one query for 64 keys, requested early: nine aligned 16-byte words that cover the 128 bytes (a row of
 // the bias starts at any even address: its length is the prompt's).  Only words that hold a bias this query needs are
-// read - keys up to min(i, key0 + 63) - so nothing past the tensor is touched; the others count as zero.  40 heads, 2 x 701
-// tokens: 60 us, against 138 with 64 two-byte loads a thread, each touching 32 rows.
+// read - keys up to min(i, key0 + 63); the others count as zero.  A word at either end may hold up to 14 bytes that are not
+// this row's, at the ends of the tensor not the tensor's; they lie in the same aligned 16 bytes as one of its values, so
+// in the same page, and are masked or shifted out.  40 heads, 2 x 701 tokens: 60 us, against 138 with 64 two-byte loads a thread, each touching 32 rows.
 struct PtBias {
     uint32_t w[36];
     uint32_t shift;   // bytes from w[0] to the first bias
