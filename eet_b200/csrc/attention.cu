@@ -95,7 +95,6 @@ struct AttnSmem {
     // copy of this structure through distributed shared memory
     float c_acc[8][128];
     float c_ml[8][2];
-    uint32_t sink[kAttnConsumerWarps];   // see reads_returned
     volatile int abort;
 };
 
@@ -291,9 +290,8 @@ decode_mha_kernel(DecodeAttnArgs a)
                 words ^= kv[u].x ^ vv[u].x;
             }
             // the tile's bytes are in registers: hand the stage back to the producer
-            reads_returned(words, &sm.sink[warp]);
             __syncwarp();
-            if ((tid & 31) == 0) mbar_arrive(&sm.empty[s]);
+            if ((tid & 31) == 0) mbar_arrive_after(&sm.empty[s], after_reads(words, a.zero));
             // the U time steps of this half-warp are folded into the running softmax together: independent
             // dot products and shuffle chains, one rescale of the accumulators per tile
             float sc[U];

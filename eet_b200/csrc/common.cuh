@@ -118,12 +118,17 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 // Before a warp hands a shared-memory stage back to the copy engine, its reads of the stage must have returned.  An mbarrier
 // arrival does not wait for them: reads held up behind another kernel's memory traffic on the same SM (under programmatic
 // dependent launch the preceding kernel's last CTAs) were passed by the arrival and saw the next copy's bytes, in 1 of 100
-// calls of the stream-K GEMM behind a finishing launch.  Instructions issue in order, and a store that needs a word of every
-// read cannot issue before they have returned, so the arrival behind it cannot either.  `words`: one word of each read,
-// combined; `sink`: a word that nobody reads.
-__device__ __forceinline__ void reads_returned(uint32_t words, uint32_t* sink)
+// calls of the stream-K GEMM behind a finishing launch.  So the request or arrival that lets the stage go takes its address
+// from the reads: `words` combines one word of each, `zero` is a kernel argument that is always 0, and an instruction cannot
+// issue before its operands are there.
+__device__ __forceinline__ uint32_t after_reads(uint32_t words, uint32_t zero)
 {
-    asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_u32(sink)), "r"(words) : "memory");
+    return words & zero;
+}
+
+__device__ __forceinline__ void mbar_arrive_after(uint64_t* bar, uint32_t offset)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar) + offset) : "memory");
 }
 
 // 1-D bulk copy global -> shared through the TMA engine; completion is signalled on `bar` as

@@ -67,7 +67,6 @@ struct MidSmem {
     uint64_t h_ready[kMidNHMax], h_empty[kMidNHMax];    // fp16 weights written (4 warps) / their MMAs completed
     uint64_t acc_full[2];                               // all MMAs of a strip segment have completed
     uint64_t acc_empty[2];                              // the epilogue warps have read the accumulator buffer (4 warps)
-    uint32_t sink[4];                                   // see reads_returned
     uint32_t tmem_base;
     volatile int abort;
 };
@@ -310,9 +309,8 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, GemmArgs a)
                 }
             }
             // the int8 stage is free again as soon as the bytes are in registers
-            reads_returned(words, &sm.sink[warp & 3]);
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.w_empty[sw]);
+            if (lane == 0) mbar_arrive_after(&sm.w_empty[sw], after_reads(words, a.zero));
             bool live = true;
 #pragma unroll
             for (int kk = 0; kk < kMidUnitK; ++kk) {

@@ -64,7 +64,6 @@ gemm_row_kernel(RowGemmArgs a)
 {
     extern __shared__ __align__(128) uint8_t row_dyn[];   // [warp][slot] tiles | partial sums of the other ranks
     __shared__ uint64_t full[kRowWarps][kRowSlots];
-    __shared__ uint32_t sink[kRowWarps];                  // see reads_returned
     pdl_launch_dependents();
     constexpr int kMats = kPair ? 2 : 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -76,15 +75,15 @@ gemm_row_kernel(RowGemmArgs a)
 
     // ---- this warp's ring: tiles warp, warp + 8, ... of the share, of both matrices in turn ----
     const int mine = n_tiles > warp ? (n_tiles - warp + kRowWarps - 1) / kRowWarps : 0;
-    auto issue = [&](int q, int slot) {
+    auto issue = [&](int q, int slot, uint32_t offset) {
         const int i = warp + kRowWarps * (q / kMats);
         mbar_arrive_expect_tx(&full[warp][slot], kTileBytes);
-        bulk_g2s_stream(ring + slot * kTileBytes, (q % kMats ? a.B2 : a.B) + first + (size_t)i * kTileBytes, kTileBytes, &full[warp][slot]);
+        bulk_g2s_stream(ring + slot * kTileBytes, (q % kMats ? a.B2 : a.B) + first + (size_t)i * kTileBytes + offset, kTileBytes, &full[warp][slot]);
     };
     if (lane == 0) {
         for (int s = 0; s < kRowSlots; ++s) mbar_init(&full[warp][s], 1);
         mbar_fence_init();
-        for (int s = 0; s < kRowSlots && s < kMats * mine; ++s) issue(s, s);
+        for (int s = 0; s < kRowSlots && s < kMats * mine; ++s) issue(s, s, 0);
     }
     __syncwarp();
     if (S > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // waited for before the first remote store
@@ -195,7 +194,7 @@ gemm_row_kernel(RowGemmArgs a)
                 const uint4 wb = *reinterpret_cast<const uint4*>(w + cg * 1024 + 512);
                 const uint32_t wa4[4] = {wa.x, wa.y, wa.z, wa.w};
                 const uint32_t wb4[4] = {wb.x, wb.y, wb.z, wb.w};
-                words = wb.w;   // (a warp's reads return in order)
+                words = wb.w;   // (the reads before this one have become operands of the MMAs)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     uint32_t a0, a1, a2, a3;
@@ -207,10 +206,9 @@ gemm_row_kernel(RowGemmArgs a)
                     }
                 }
             }
-            reads_returned(words, &sink[warp]);
             __syncwarp();
             const int q = kMats * j + p + kRowSlots;
-            if (lane == 0 && live && q < kMats * mine) issue(q, slot);
+            if (lane == 0 && live && q < kMats * mine) issue(q, slot, after_reads(words, a.zero));
             if (++slot == kRowSlots) {
                 slot = 0;
                 phase ^= 1;

@@ -67,7 +67,6 @@ struct SkinnySmem {
     uint64_t full[kMaxStages];
     uint64_t empty[kMaxStages];
     float fold[4][2][32][4];  // fragments of warps 4-7 on their way to warps 0-3 at the end of a tile row
-    uint32_t sink[kConsumerWarps];   // see reads_returned
     volatile int abort;
 };
 
@@ -251,7 +250,7 @@ gemm_skinny_kernel(GemmArgs a)
                 }
                 const uint4 wa = *reinterpret_cast<const uint4*>(ws + tile * kTileBytes);
                 const uint4 wb = *reinterpret_cast<const uint4*>(ws + tile * kTileBytes + 512);
-                words = wb.w;   // (a warp's reads return in order)
+                words = wb.w;   // (the reads before this one have become operands of the MMAs)
                 const uint32_t wa4[4] = {wa.x, wa.y, wa.z, wa.w};
                 const uint32_t wb4[4] = {wb.x, wb.y, wb.z, wb.w};
 #pragma unroll
@@ -266,9 +265,8 @@ gemm_skinny_kernel(GemmArgs a)
                 }
             }
         }
-        reads_returned(words, &sm.sink[warp]);
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.empty[s]);
+        if (lane == 0) mbar_arrive_after(&sm.empty[s], after_reads(words, a.zero));
         g += nb_tiles;
 
         const bool row_end = (kb + nb_tiles == KT);

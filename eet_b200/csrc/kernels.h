@@ -24,6 +24,7 @@ struct GemmArgs {
     float* ws;          // [M][N] fp32: sum over k of A[m][k] * q[k][n] is ADDED here
     float* ws2;         // the same for B2
     int M, N, K;
+    uint32_t zero;      // 0, see after_reads
 };
 size_t skinny_sum_bytes(int M, int N);
 int launch_gemm_skinny(const GemmArgs& a, cudaStream_t stream);
@@ -45,6 +46,7 @@ struct RowGemmArgs {
     float eps;
     int M, N, K, gate;
     int splits;              // CTAs per tile row, chosen by the launcher
+    uint32_t zero;           // 0, see after_reads
 };
 bool gemm_row_wastes_a_wave(int M, int N, int K);   // the skinny kernel is the faster one
 int launch_gemm_row(RowGemmArgs a, cudaStream_t stream);
@@ -121,6 +123,7 @@ struct DecodeAttnArgs {
     int rope;                 // 1: rotate q,k (NeoX pairing) at position step-1
     float rope_base;
     int splits;               // CTAs per (batch, head): 1, 2, 4 or 8; 0 = choose
+    uint32_t zero;            // 0, see after_reads
 };
 struct AttnPlan {
     int splits, ctas;   // CTAs per (batch, head) pair, CTAs per SM
