@@ -15,6 +15,8 @@ Additions that the reference does not have, all optional: `tp` (a tensor-paralle
 eet_b200.tp) on MetaDesc, and device-resident step counters so that a decode step can be replayed as a
 CUDA graph (eet_b200.modeling).
 """
+import ctypes
+import functools
 import math
 
 import torch
@@ -292,7 +294,8 @@ def gemm_w8a16(x, packed_w, scale, out=None, residual=None, gate=None):
         out = torch.empty((M, N), dtype=torch.float16, device=x.device)
     if gate is not None and residual is not None:
         raise RuntimeError("gemm_w8a16: residual and gate exclude each other")
-    if 0 < M <= _ROW_MAX_M and N <= _ROW_MAX_N and not in_place and gate is None and (residual is None or residual.numel() > 0):
+    if (0 < M <= _ROW_MAX_M and gate is None and not in_place and (residual is None or residual.numel() > 0)
+            and (N <= _ROW_MAX_N or _row_kernel_takes(M, N, K))):
         return _gemm_row(x, packed_w, scale, out, M, residual=residual)
     second, epilogue = (gate, 2) if gate is not None else (residual, 1 if residual is not None else 0)
     ws_bytes = lib.eet_gemm_w8a16_workspace_bytes(M, N, K)
@@ -303,7 +306,14 @@ def gemm_w8a16(x, packed_w, scale, out=None, residual=None, gate=None):
 
 
 _ROW_MAX_M = 16      # rows of the decode GEMM that finishes its product itself
-_ROW_MAX_N = 16384   # wider matrices may be read faster by two launches with scratch: eet_gemm_w8a16 knows
+_ROW_MAX_N = 16384   # wider matrices may be read faster by two launches with scratch
+
+
+@functools.lru_cache(maxsize=256)
+def _row_kernel_takes(M, N, K):
+    plan = (ctypes.c_int * 5)()
+    check(lib.eet_gemm_w8a16_plan(M, N, K, plan))
+    return plan[0] == 1
 
 
 def _gemm_row(x, w, scale, out, M, w2=None, scale2=None, residual=None, norm=None, squares_out=None):
