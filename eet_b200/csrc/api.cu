@@ -213,21 +213,23 @@ enum { kRouteShares = 0, kRouteRow = 1, kRouteStreamK = 2, kRouteTiles = 3, kRou
 
 struct GemmRoute {
     int kernel;
-    bool scratch;     // a caller has to bring the fp32 sums: hangs on the shape alone, whichever kernel is chosen
+    bool sums;        // sums in the scratch, finished by another launch, are a way for this shape, chosen or not
     Tc2Plan tc;
     PairPlan pair;
 };
 
-static GemmRoute gemm_route(int M, int N, int K)
+static GemmRoute gemm_route(int M, int N, int K, bool scratch)
 {
     GemmRoute r = {kRouteShares, true, Tc2Plan{0, 0, 0, 1, 1e30}, PairPlan{0, 1e30}};
     if (M <= kRowMaxM) {
         if (!gemm_row_wastes_a_wave(M, N, K)) r.kernel = kRouteRow;
         return r;
     }
-    const bool sums = M <= mid_use_max_m() && gemm_mid_supported(M, N, K) && !gemm_tc_owns(M, N, K);
-    double least = sums ? gemm_mid_us(M, N, K) : 1e30;
-    if (sums) r.kernel = kRouteStreamK;
+    r.sums = M <= mid_use_max_m() && gemm_mid_supported(M, N, K) && !gemm_tc_owns(M, N, K);
+    // (a caller without scratch gets tiles where they can take the shape)
+    const bool stream_k = r.sums && (scratch || !gemm_tc_supported(M, N, K));
+    double least = stream_k ? gemm_mid_us(M, N, K) : 1e30;
+    if (stream_k) r.kernel = kRouteStreamK;
     r.tc = gemm_tc_plan(M, N, K);
     r.pair = gemm_pair_plan(M, N, K);
     if (r.tc.us < least) {
@@ -235,7 +237,7 @@ static GemmRoute gemm_route(int M, int N, int K)
         least = r.tc.us;
     }
     if (r.pair.us < least) r.kernel = kRoutePairs;
-    r.scratch = sums || r.kernel == kRouteShares;
+    r.sums = r.sums || r.kernel == kRouteShares;
     return r;
 }
 
@@ -243,7 +245,7 @@ int eet_gemm_w8a16_plan(int M, int N, int K, int* plan)
 {
     if (check_kn("eet_gemm_w8a16_plan", K, N)) return 1;
     EET_CHECK(M > 0 && plan != nullptr, "eet_gemm_w8a16_plan: M must be positive and plan not NULL");
-    const GemmRoute r = gemm_route(M, N, K);
+    const GemmRoute r = gemm_route(M, N, K, true);
     plan[0] = r.kernel;
     plan[1] = r.kernel == kRouteTiles ? r.tc.bn : (r.kernel == kRoutePairs ? 2 * r.pair.bn : 0);
     plan[2] = r.kernel == kRouteTiles ? r.tc.whole : 0;
@@ -263,15 +265,17 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
               "eet_gemm_w8a16: epilogues 1 and 2 need a 16-byte aligned second operand");
     const __half* res = epilogue != 0 ? (const __half*)residual : nullptr;
     const int gate = epilogue == 2 ? 1 : 0;
-    GemmRoute route = gemm_route(M, N, K);
-    EET_CHECK(!route.scratch || (ws && aligned16(ws) && ws_bytes >= eet_gemm_w8a16_workspace_bytes(M, N, K)),
-              "eet_gemm_w8a16: workspace of %zu bytes is smaller than the %zu needed", ws_bytes,
-              eet_gemm_w8a16_workspace_bytes(M, N, K));
+    const bool scratch = ws && aligned16(ws) && ws_bytes >= eet_gemm_w8a16_workspace_bytes(M, N, K);
+    GemmRoute route = gemm_route(M, N, K, scratch);
     // C over A: only sums that are finished by another launch let all of A be read before C is stored
     const uintptr_t a0 = (uintptr_t)A, a1 = a0 + (size_t)M * K * 2, c0 = (uintptr_t)C, c1 = c0 + (size_t)M * N * 2;
-    if (route.scratch && a0 < c1 && c0 < a1) route.kernel = gemm_mid_supported(M, N, K) ? kRouteStreamK : kRouteShares;
+    if (route.sums && a0 < c1 && c0 < a1) route.kernel = gemm_mid_supported(M, N, K) ? kRouteStreamK : kRouteShares;
+    // (up to 16 rows this entry point has always asked for it, whichever kernel serves)
+    EET_CHECK(scratch || (M > kRowMaxM && route.kernel != kRouteStreamK && route.kernel != kRouteShares),
+              "eet_gemm_w8a16: workspace of %zu bytes is smaller than the %zu needed", ws_bytes,
+              eet_gemm_w8a16_workspace_bytes(M, N, K));
     if (route.kernel == kRouteRow) {
-        // decode regime: one launch that leaves the scratch alone (this entry point has always asked for it)
+        // decode regime: one launch that leaves the scratch alone
         RowGemmArgs r = {};
         r.A = (const __half*)A;
         r.B = (const uint8_t*)packedB;

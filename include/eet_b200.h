@@ -107,15 +107,16 @@ size_t eet_gemm_w8a16_workspace_bytes(int M, int N, int K);
  *             called from csrc/op/gated_ffn_int8.cpp:290-301) fused in, with its mix of fp32 and fp16 arithmetic.
  *   residual  device fp16 [M][N] for epilogues 1 and 2, else NULL (may alias C)
  * M may be any value >= 0; K and N must be multiples of 64; pointers 16-byte aligned.  C may lie over A up to 64 rows, and up
- * to 512 for shapes that need the scratch.
+ * to 512 for narrow shapes (below), with scratch.
  * Kernels: M <= 16 the row kernel (one launch, leaves the scratch alone), wide matrices that would leave its last wave
  * mostly empty the equal-share kernel into the scratch with a finishing launch; 16 < M <= 64 (N % 128 == 0) stream-K
  * into the scratch with a finishing launch; above that the shortest of three modelled times decides between stream-K (up
  * to 512 rows), tiles of 256 channels on single CTAs or with the reduction split over clusters of 2-4, and tiles on CTA
  * pairs (from 256 rows); shapes with N % 128 == 64 take the equal-share kernel in groups of 128 rows.
- * Scratch is needed for M <= 64, for N % 128 == 64, and up to 512 rows for narrow shapes: N % 256 != 0, or 256 x 256 tiles
- * so few that not 96 CTAs (120 without a split) would share them.  The others go to tiles whatever the models say and
- * give the same bits every time; stream-K and equal shares add in the order of arrival.
+ * Scratch is needed for M <= 64, for N % 128 == 64, and for C over A.  Up to 512 rows, narrow shapes (N % 256 != 0, or
+ * 256 x 256 tiles so few that not 96 CTAs, or 120 without a split, would share them) use it where that is faster and go
+ * to tiles without it; the others always go to tiles.  Tiles and the row kernel give the same bits every time, stream-K
+ * and equal shares add in the order of arrival.
  */
 int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* C, int M, int N, int K,
                    const void* residual, int epilogue, void* ws, size_t ws_bytes, void* stream);

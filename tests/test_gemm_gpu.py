@@ -377,7 +377,7 @@ def test_baichuan13b_and_llama65b_projection_shapes(KN):
                                    (5120, 5120, 384), (8192, 3072, 512), (1088, 6144, 300)])
 def test_wide_shapes_repeat_bit_for_bit_and_need_no_scratch(K, N, M):
     """From 65 rows on, shapes with enough 256-channel tiles (whole, or split over clusters): the same bits every time, and no
-    scratch.  Narrow ones sum in global memory: without scratch they are refused."""
+    scratch.  Narrow ones may sum in global memory; without scratch they run on tiles, and with 40 rows they are refused."""
     from eet_b200._lib import check, lib
     from eet_b200 import EET
     gen = torch.Generator(device="cuda").manual_seed(M)
@@ -387,9 +387,9 @@ def test_wide_shapes_repeat_bit_for_bit_and_need_no_scratch(K, N, M):
     packed = EET.preprocess_weights(q)
     stream = torch.cuda.current_stream().cuda_stream
 
-    def call(w, n):
-        out = torch.empty(M, n, dtype=torch.float16, device="cuda")
-        rc = lib.eet_gemm_w8a16(x.data_ptr(), w.data_ptr(), s.data_ptr(), out.data_ptr(), M, n, K, None, 0, None, 0, stream)
+    def call(w, n, rows=M):
+        out = torch.empty(rows, n, dtype=torch.float16, device="cuda")
+        rc = lib.eet_gemm_w8a16(x.data_ptr(), w.data_ptr(), s.data_ptr(), out.data_ptr(), rows, n, K, None, 0, None, 0, stream)
         return rc, out
     rc, first = call(packed, N)
     check(rc)
@@ -397,7 +397,12 @@ def test_wide_shapes_repeat_bit_for_bit_and_need_no_scratch(K, N, M):
     assert ((first.double() - y).abs() <= 2.0 ** -10 * y.abs() + 1e-4).all()   # one rounding to fp16, doubled
     for _ in range(8):
         assert torch.equal(call(packed, N)[1], first)
-    assert call(EET.preprocess_weights(q[:, :128].contiguous()), 128)[0] != 0 and b"workspace" in lib.eet_last_error()
+    narrow = EET.preprocess_weights(q[:, :128].contiguous())
+    rc, part = call(narrow, 128)
+    check(rc)
+    assert ((part.double() - y[:, :128]).abs() <= 2.0 ** -10 * y[:, :128].abs() + 1e-4).all()
+    for rows in (1, 16, 40, 64):
+        assert call(narrow, 128, rows)[0] != 0 and b"workspace" in lib.eet_last_error()
 
 
 @pytest.mark.parametrize("M", [17, 32, 40, 64, 100, 128, 250, 256, 400, 512])
