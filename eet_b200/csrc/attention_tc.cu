@@ -20,17 +20,22 @@
 //                      TENSOR MEMORY as the A operand and V straight from its [key][dim] tile as an MN-major B
 //                      operand - V is never transposed and P never touches shared memory.
 //   warps 2-5          softmax, one thread per query row (= TMEM lane): tcgen05.ld of the row's 64 scores,
-//                      scale / fp16 rounding / bias / masks, running max and sum, probabilities back INTO THE
+//                      scale / bias / masks, running max and sum, probabilities back INTO THE
 //                      SCORE COLUMNS as fp16 pairs (tcgen05.st: a row only ever touches its own lane, and the
 //                      tensor core overwrites a score buffer only after the P.V that read it, in issue order);
-//                      the O accumulator is rescaled only when some row of the warp saw a new maximum.  At the
-//                      end they read O, normalise and store the context.
+//                      the O accumulator is rescaled only when a row's maximum has outgrown the one that O is
+//                      accumulated under by 2^8.  At the end they read O, normalise and store the context.
 // Every wait is bounded (device status 2) and the CTA frees its tensor memory on every path.
 //
 // Numerics kept from the reference and from the mma.sync kernel this one replaces for long prompts: scores scaled
-// by the fp16-rounded 1/sqrt(D) and rounded to fp16 where the reference stores them in fp16, the ALiBi bias added
-// in fp32 after that rounding, probabilities enter P.V as fp16, denominator + 1e-6, rows above the left padding
-// are zero.
+// by the fp16-rounded 1/sqrt(D), the ALiBi bias added in fp32, probabilities enter P.V as fp16, denominator + 1e-6, rows
+// above the left padding are zero.  The scores stay in fp32: the reference stores them as fp16, which costs more than half of
+// the error of the result (relative to 64 bits 4.4e-4 with that rounding, 2.6e-4 without it, 2 x 2048 tokens).
+//
+// Measured, 32 heads: 2 x 2048 tokens 89 us (138 with a rescale of O in nearly every block, one chain of 64 maxima, the
+// tiles of a pair behind one another and the fp16 rounding), 8 x 512 48 us (58); 40 heads with a bias, 2 x 701 tokens 41 us
+// (56).  Time stamps: a block takes 1650 cycles on each of an SM's two CTAs, and the issuing thread is the one that never waits: Q.K^T
+// with 64 keys reads 6 KiB of shared memory per MMA (48 cycles) for 32 cycles of multiplications.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -81,18 +86,6 @@ __device__ __forceinline__ float ex2_approx(float x)
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-
-// x rounded to the 11 significant bits of an fp16 value, in fp32 arithmetic (Veltkamp's splitting: three FP32
-// operations instead of a conversion to half and back - the conversion unit is the one that also evaluates the
-// exponentials, and it is what bounds the softmax).  Equal to fp16(x) for |x| inside fp16's normal range except
-// on exact ties, where it may pick the other neighbour; scores outside that range (|x| < 6e-5) keep more bits
-// than fp16 would, which no softmax can see.
-__device__ __forceinline__ float round_to_half_precision(float x)
-{
-    // (intrinsics: the compiler must not contract these into fused multiply-adds, which would skip a rounding)
-    const float big = __fmul_rn(x, 8193.0f);   // 2^13 + 1
-    return __fsub_rn(big, __fsub_rn(big, x));
 }
 
 // B operand held [k][n] with n contiguous (MN-major), 128-byte swizzle: 64 n-values per 128-byte row, 8 k-rows per
@@ -146,10 +139,88 @@ struct PtBias {
     }
 };
 
+// 32 columns of tensor memory into 32 registers, without waiting for them
+__device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, uint32_t* v)
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr));
+}
+
+// (the registers pass through the wait, so that nothing reads them above it)
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&v)[kPtK])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int c = 0; c < kPtK; ++c) asm volatile("" : "+r"(v[c]));
+}
+
+// The FP32 operations of the softmax, two scores at a time (one instruction for a pair of registers).
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t pair2(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 split2(uint64_t v)
+{
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
+
+__device__ __forceinline__ float max3(float a, float b, float c)
+{
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// exp(s - m) of a row's 64 scores as one FMA and one ex2 each (-inf stays -inf and gives 0), as fp16 pairs; returns their sum
+__device__ __forceinline__ float exponentials(const uint64_t (&sc)[kPtK / 2], float to_log2, float m, uint32_t (&pk)[kPtK / 2])
+{
+    const uint64_t to_log2_2 = pair2(to_log2, to_log2), m_l2 = pair2(-m * to_log2, -m * to_log2);
+    uint64_t psum[2] = {0ull, 0ull};
+#pragma unroll
+    for (int c = 0; c < kPtK / 2; ++c) {
+        const float2 e = split2(fma2(sc[c], to_log2_2, m_l2));
+        const float p0 = ex2_approx(e.x), p1 = ex2_approx(e.y);
+        psum[c & 1] = add2(psum[c & 1], pair2(p0, p1));
+        const __half2 hp = __floats2half2_rn(p0, p1);
+        pk[c] = *reinterpret_cast<const uint32_t*>(&hp);
+    }
+    const float2 ps = split2(add2(psum[0], psum[1]));
+    return ps.x + ps.y;
+}
+
 template<bool kBias>
 __global__ void __launch_bounds__(kPtThreads, 2)
 prefill_mha_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                      const __grid_constant__ CUtensorMap map_v, __half* __restrict__ ctx, int S, int H,
+                      const __grid_constant__ CUtensorMap map_v, __half* __restrict__ ctx, int S, int H, int heads, int group,
                       const int64_t* __restrict__ pad_len, const __half* __restrict__ alibi, int alibi_stride)
 {
     constexpr int D = 128;
@@ -160,10 +231,16 @@ prefill_mha_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     uint8_t* k_ring = q_tile + kPtQTile;
     uint8_t* v_ring = k_ring + kPtStages * kPtKvTile;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int bh = blockIdx.y;
+    // Tiles in the order of their length, the longest (late queries) of all (batch, head) pairs of a group first, so that
+    // short ones fill the end: with the tiles of one pair behind another a pair's longest tile began last.
+    // A group is as many pairs as fit the L2 with their keys and values.
+    const int q_tiles = (S + kPtQ - 1) / kPtQ;
+    const int first_pair = (int)blockIdx.x / (q_tiles * group) * group;
+    const int in_group = min(group, heads - first_pair);
+    const int place = (int)blockIdx.x - first_pair * q_tiles;
+    const int bh = first_pair + place % in_group;
     const int b = bh / H, h = bh % H;
-    const int qb = (int)gridDim.x - 1 - (int)blockIdx.x;   // the long tiles (late queries) are scheduled first
-    const int i0 = qb * kPtQ;
+    const int i0 = (q_tiles - 1 - place / in_group) * kPtQ;
     const int pad = (pad_len != nullptr && alibi == nullptr) ? (int)pad_len[b] : 0;
     const int kb_first = pad / kPtK;                                        // key blocks left of the padding are skipped
     const int kb_last = min((i0 + kPtQ - 1) / kPtK, (S - 1) / kPtK);        // causal: nothing above the diagonal
@@ -281,7 +358,13 @@ prefill_mha_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         const int i = i0 + r;
         const uint32_t t_lane = (uint32_t)lane_base << 16;
         const float scalar = __half2float(__float2half(sqrtf(1.0f / D)));
-        float m_run = -1e20f, l_run = 0.f;
+        const uint64_t scalar2 = pair2(scalar, scalar);
+        // From the scores as they are kept (scaled already with a bias, straight from the accumulator without) to powers of 2.
+        const float to_log2 = kBias ? 1.4426950408889634f : 1.4426950408889634f * scalar;
+        // m_ref: the maximum under which O and l_run are accumulated.  It follows the running maximum m_run only when that
+        // has outgrown it by 2^8: until then the probabilities are at most 256, which fp16 holds as exactly as those
+        // up to 1, and the common factor leaves with the division at the end.
+        float m_run = -1e20f, m_ref = -1e20f, l_run = 0.f;
         const __half* arow = kBias ? alibi + ((size_t)h * alibi_stride + (i < S ? i : 0)) * alibi_stride : nullptr;
         bool ok = n_blocks > 0;
         for (int jl = 0; jl < n_blocks && ok; ++jl) {
@@ -289,99 +372,72 @@ prefill_mha_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             PtBias bias;
             if (kBias) bias.load(arow, key0, i, i < S);   // on its way while the scores are computed
             const uint32_t t_s = tmem + t_lane + kPtColS + (uint32_t)((jl & 1) * kPtK);   // this block's score buffer
-            int got = 1;
-            if (lane == 0) got = tc_wait(&sm.s_full[jl & 1], (uint32_t)((jl >> 1) & 1), &sm.abort) ? 1 : 0;
-            got = __shfl_sync(0xffffffffu, got, 0);
-            if (!got) {
+            if (!tc_wait_warp(&sm.s_full[jl & 1], (uint32_t)((jl >> 1) & 1), &sm.abort)) {
                 ok = false;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            float sc[kPtK];
+            uint64_t sc[kPtK / 2];
+            {
+                uint32_t v[kPtK];
+                tmem_ld32_async(t_s, v);
+                tmem_ld32_async(t_s + 32, v + 32);
+                if (kBias) bias.align();
+                tmem_ld_wait(v);
 #pragma unroll
-            for (int c0 = 0; c0 < kPtK; c0 += 32) {
-                uint32_t v[32];
-                tmem_ld32(t_s + (uint32_t)c0, v);
-#pragma unroll
-                for (int c = 0; c < 32; ++c) sc[c0 + c] = __uint_as_float(v[c]);
+                for (int c = 0; c < kPtK / 2; ++c) sc[c] = pair2(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1]));
             }
-
-            float mx = -INFINITY;
-            // a block left of the diagonal, right of the padding and inside the prompt needs no per-element mask
-            const bool whole = (key0 + kPtK - 1 <= i) && (key0 >= pad) && (key0 + kPtK <= S);
             if (kBias) {
-                bias.align();
 #pragma unroll
-                for (int c = 0; c < kPtK; c += 2) {
-                    const float2 b2 = __half22float2(*reinterpret_cast<const __half2*>(&bias.w[c >> 1]));
-                    sc[c] = round_to_half_precision(sc[c] * scalar) + b2.x;
-                    sc[c + 1] = round_to_half_precision(sc[c + 1] * scalar) + b2.y;
+                for (int c = 0; c < kPtK / 2; ++c) {
+                    const float2 b2 = __half22float2(*reinterpret_cast<const __half2*>(&bias.w[c]));
+                    sc[c] = fma2(sc[c], scalar2, pair2(b2.x, b2.y));
                 }
             }
-            else {
+            // a block left of the diagonal of all rows of the warp, right of the padding and inside the prompt needs no mask
+            if (!((key0 + kPtK - 1 <= i0 + lane_base) && (key0 >= pad) && (key0 + kPtK <= S))) {
 #pragma unroll
-                for (int c = 0; c < kPtK; ++c) sc[c] = round_to_half_precision(sc[c] * scalar);
-            }
-            if (whole) {
-#pragma unroll
-                for (int c = 0; c < kPtK; ++c) mx = fmaxf(mx, sc[c]);
-            }
-            else {
-#pragma unroll
-                for (int c = 0; c < kPtK; ++c) {
-                    const int j = key0 + c;
-                    sc[c] = (j <= i && j >= pad && j < S) ? sc[c] : -INFINITY;
-                    mx = fmaxf(mx, sc[c]);
+                for (int c = 0; c < kPtK / 2; ++c) {
+                    const int j = key0 + 2 * c;
+                    float2 f = split2(sc[c]);
+                    f.x = (j <= i && j >= pad && j < S) ? f.x : -INFINITY;
+                    f.y = (j + 1 <= i && j + 1 >= pad && j + 1 < S) ? f.y : -INFINITY;
+                    sc[c] = pair2(f.x, f.y);
                 }
             }
-            constexpr float kLog2e = 1.4426950408889634f;
-            const float m_new = fmaxf(m_run, mx);
-            const float corr = ex2_approx((m_run - m_new) * kLog2e);
-            m_run = m_new;
-            const float m_l2 = -m_new * kLog2e;
-            float psum = 0.f;
+            // (four chains side by side: one of 64 dependent maxima took as long as the exponentials)
+            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int c = 0; c < kPtK / 2; ++c) {
+                const float2 f = split2(sc[c]);
+                mx[c & 3] = max3(mx[c & 3], f.x, f.y);
+            }
+            m_run = fmaxf(m_run, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
+            float corr = 1.0f;
+            const bool moves = (m_run - m_ref) * to_log2 > 8.0f;
+            if (moves) {
+                corr = ex2_approx((m_ref - m_run) * to_log2);
+                m_ref = m_run;
+            }
             uint32_t pk[kPtK / 2];
-#pragma unroll
-            for (int c = 0; c < kPtK; c += 2) {
-                // exp(s - m) as one FMA and one ex2 (-inf stays -inf and gives 0)
-                const float p0 = ex2_approx(fmaf(sc[c], kLog2e, m_l2)), p1 = ex2_approx(fmaf(sc[c + 1], kLog2e, m_l2));
-                psum += p0 + p1;
-                const __half2 hp = __floats2half2_rn(p0, p1);
-                pk[c >> 1] = *reinterpret_cast<const uint32_t*>(&hp);
-            }
-            l_run = l_run * corr + psum;
+            l_run = l_run * corr + exponentials(sc, to_log2, m_ref, pk);
             // probabilities as the A operand of P.V: lane = query, 16-bit pairs along the columns, written over the
             // first half of this row's scores (which are in registers by now)
-            {
-                uint32_t v[32];
-#pragma unroll
-                for (int c0 = 0; c0 < kPtK / 2; c0 += 32) {
-#pragma unroll
-                    for (int c = 0; c < 32; ++c) v[c] = pk[c0 + c];
-                    tmem_st32(t_s + (uint32_t)c0, v);
+            tmem_st32(t_s, pk);
+            // rescale O where a row of this warp has moved its reference, after the previous block's P.V has completed
+            if (jl > 0 && __any_sync(0xffffffffu, moves)) {
+                if (!tc_wait_warp(&sm.pv_done[(jl - 1) & 1], (uint32_t)(((jl - 1) >> 1) & 1), &sm.abort)) {
+                    ok = false;
+                    break;
                 }
-            }
-            // O accumulates under the old maximum: rescale it if any row of this warp moved, after the previous
-            // block's P.V has completed
-            if (jl > 0) {
-                const unsigned moved = __ballot_sync(0xffffffffu, corr != 1.0f);
-                if (moved != 0u) {
-                    int done = 1;
-                    if (lane == 0) done = tc_wait(&sm.pv_done[(jl - 1) & 1], (uint32_t)(((jl - 1) >> 1) & 1), &sm.abort) ? 1 : 0;
-                    done = __shfl_sync(0xffffffffu, done, 0);
-                    if (!done) {
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-                    for (int c0 = 0; c0 < D; c0 += 32) {
-                        uint32_t v[32];
-                        tmem_ld32(tmem + t_lane + kPtColO + (uint32_t)c0, v);
+                for (int c0 = 0; c0 < D; c0 += 32) {
+                    uint32_t v[32];
+                    tmem_ld32(tmem + t_lane + kPtColO + (uint32_t)c0, v);
 #pragma unroll
-                        for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) * corr);
-                        tmem_st32(tmem + t_lane + kPtColO + (uint32_t)c0, v);
-                    }
+                    for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) * corr);
+                    tmem_st32(tmem + t_lane + kPtColO + (uint32_t)c0, v);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -410,7 +466,7 @@ prefill_mha_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         if (n_blocks > 0 && ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // rows above the left padding are zeroed by the reference (gpt2_self_softmax.cu:24-30)
-            const float inv = (i < pad) ? 0.f : 1.0f / (l_run + 1e-6f);
+            const float inv = (i < pad) ? 0.f : 1.0f / (l_run + 1e-6f * ex2_approx((m_run - m_ref) * to_log2));
 #pragma unroll 1
             for (int c0 = 0; c0 < D; c0 += 32) {
                 uint32_t v[32];
@@ -461,6 +517,7 @@ int encode_rows_map(CUtensorMap* map, const __half* basep, int rows, size_t rows
 
 // Prompts of at least this many tokens go to the tensor-core kernel (its tiles are 128 queries x 64 keys).
 constexpr int kPrefillTcMinS = 96;
+constexpr long long kPtGroupBytes = 64ll << 20;   // keys and values that are worked on at a time: half of the L2
 
 bool prefill_mha_tc_supported(int S, int D)
 {
@@ -484,8 +541,11 @@ int launch_prefill_mha_tc(const __half* q, const __half* kcache, const __half* v
         EET_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPtSmem));
         attr_set[dev][alibi != nullptr] = true;
     }
-    dim3 grid((S + kPtQ - 1) / kPtQ, B * H);
-    kern<<<grid, kPtThreads, kPtSmem, stream>>>(map_q, map_k, map_v, ctx, S, H, pad_len, alibi, alibi_stride);
+    const long long blocks = (long long)((S + kPtQ - 1) / kPtQ) * B * H;
+    EET_CHECK(blocks <= 0x7fffffffLL, "prefill attention: %lld tiles exceed the grid limit", blocks);
+    const long long fit = kPtGroupBytes / ((long long)S * 512);   // K and V of a pair: 512 bytes a token
+    const int group = fit < 1 ? 1 : (fit < B * H ? (int)fit : B * H);
+    kern<<<(unsigned)blocks, kPtThreads, kPtSmem, stream>>>(map_q, map_k, map_v, ctx, S, H, B * H, group, pad_len, alibi, alibi_stride);
     EET_LAUNCH_CHECK();
     return 0;
 }

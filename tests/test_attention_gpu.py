@@ -230,6 +230,48 @@ def test_prefill_bias_at_any_alignment(S, offset):
     assert torch.allclose(got.float(), ref.float(), atol=4e-3, rtol=4e-3)
 
 
+def _prefill64(q, k, v, bias):
+    """Causal attention of one head in 64 bits, and the same with |v|: the bound of an error that is relative to each product."""
+    S = q.shape[0]
+    scores = (q.double() @ k.double().t()) * float(torch.tensor(128 ** -0.5).half())
+    if bias is not None:
+        scores = scores + bias.double()
+    scores = scores.masked_fill(torch.triu(torch.ones(S, S, dtype=torch.bool, device=q.device), 1), float("-inf"))
+    p = torch.softmax(scores, -1)
+    return p @ v.double(), p @ v.double().abs()
+
+
+@pytest.mark.parametrize("S,B,H,mode", [(257, 1, 2, "rising"), (300, 1, 2, "steps"), (383, 1, 2, "lowest"), (1100, 1, 130, "plain"),
+                                        (2047, 2, 37, "plain")])
+def test_prefill_moving_maximum_and_pair_groups(S, B, H, mode):
+    """The softmax keeps an old reference until the maximum has outgrown it by 2^8: scores that rise a little with every block,
+    by jumps, and from fp16's lowest value; and more (batch, head) pairs than are worked on at a time (64 MiB of keys and
+    values), the last group smaller.  Probabilities and outputs are rounded once to fp16 (2^-11 relative each), scores of a few
+    hundred in fp32 move an exponential by less than 1e-4."""
+    from eet_b200._lib import check, lib
+    D = 128
+    gen = torch.Generator(device="cuda").manual_seed(S)
+    q, k, v = (torch.randn(B, H, S, D, generator=gen, device="cuda").half() for _ in range(3))
+    bias = None
+    t = torch.arange(S, device="cuda")
+    if mode == "rising":
+        bias = (0.11 * t).half().expand(H, S, S).contiguous()
+    elif mode == "steps":
+        bias = (37.0 * (t // 90)).half().expand(H, S, S).contiguous()
+    elif mode == "lowest":
+        bias = torch.where(t < 200, -65504.0, 0.0).half().expand(H, S, S).contiguous()
+    ctx = torch.empty(B, S, H, D, dtype=torch.float16, device="cuda")
+    check(lib.eet_prefill_mha(q.data_ptr(), k.data_ptr(), v.data_ptr(), ctx.data_ptr(), B, S, H, D, S, None,
+                              None if bias is None else bias.data_ptr(), S, _stream()))
+    for b, h in {(0, 0), (0, H // 2), (B - 1, H - 2), (B - 1, H - 1)}:
+        ref, size = _prefill64(q[b, h], k[b, h], v[b, h], None if bias is None else bias[h])
+        err = (ctx[b, :, h].double() - ref).abs()
+        if mode == "lowest":   # -65504 leaves a score 8 bits behind the point: up to 2^-9 in an exponent
+            assert bool((err[:200] <= 2 ** -7 * size[:200]).all())
+            err, size = err[200:], size[200:]
+        assert bool((err <= (2 ** -10 + 1e-4) * size + 2 ** -24).all())
+
+
 def test_decode_finishes_projection_sums_itself():
     """qkv given as the fp32 sums of the projection GEMM + per-channel scales: same result as the fp16 form,
     and the sums are zero afterwards."""
