@@ -251,7 +251,7 @@ prefill_mha_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         tma_load_3d(tile, map, 0, key0, bh, bar);
         tma_load_3d(tile + kPtKvHalf, map, 64, key0, bh, bar);
     };
-    if (threadIdx.x == 0) {
+    if (warp == 0 && elect_one()) {
         mbar_init(&sm.q_full, 1);
         for (int st = 0; st < kPtStages; ++st) {
             mbar_init(&sm.k_full[st], 1);
@@ -291,7 +291,7 @@ prefill_mha_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             for (int jl = kPtStages; jl < n_blocks; ++jl) {
                 const int st = jl % kPtStages;
                 const uint32_t ph = (uint32_t)((jl / kPtStages - 1) & 1);
@@ -305,7 +305,7 @@ prefill_mha_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     }
     else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0 && n_blocks > 0) {
+        if (n_blocks > 0 && elect_one()) {
             constexpr uint32_t idesc_qk = umma_idesc_f16(128, kPtK);                  // both operands K-major
             constexpr uint32_t idesc_pv = umma_idesc_f16(128, D) | (1u << 16);        // B operand MN-major
             const uint64_t q_desc = umma_desc_sw128(smem_u32(q_tile));

@@ -64,6 +64,23 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p)
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// True for one lane of the (whole) warp, always the same one.  The roles that issue TMA copies and tcgen05 instructions are one
+// thread, and it is chosen with this and not with lane == 0: these instructions take their operands from uniform registers, and
+// only behind elect.sync does the compiler know that a single thread is active.  Behind lane == 0 it serialises over the lanes
+// that might be: eight MMAs and two commits took 750 to 950 cycles to issue, against 130 to 170 behind this.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t pred;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(pred));
+    return pred != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

@@ -129,7 +129,7 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, GemmArgs a)
 
     pdl_launch_dependents();
 
-    if (threadIdx.x == 0) {
+    if (warp == 0 && elect_one()) {
         for (int s = 0; s < kMidNW; ++s) {
             mbar_init(&sm.w_full[s], 1);
             mbar_init(&sm.w_empty[s], 4);
@@ -176,7 +176,7 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, GemmArgs a)
             ++w_strip;
         }
     };
-    if (threadIdx.x == 0) {
+    if (warp == 0 && elect_one()) {
         while (w_fill < kMidNW && w_u < u1) issue_w();
     }
     if (warp == 1) {
@@ -196,7 +196,7 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, GemmArgs a)
     const uint32_t tmem = sm.tmem_base;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             while (w_u < u1) {
                 if (!tc_wait(&sm.w_empty[w_s], w_ph, &sm.abort)) break;
                 issue_w();
@@ -205,7 +205,7 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, GemmArgs a)
     }
     else if (warp == 10) {
         // ------------------------------------------------------------------ activation producer
-        if (lane == 0) {
+        if (elect_one()) {
             pdl_wait();   // the activations are the preceding kernel's output
             int s = 0, fill = 0;
             uint32_t ph = 1;
@@ -229,7 +229,7 @@ gemm_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, GemmArgs a)
     }
     else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = umma_idesc_f16(128, BN);
             const uint64_t b_desc0 = umma_desc_sw128(smem_u32(x_ring));
             const uint32_t a_tmem0 = tmem + kAColBase;

@@ -14,8 +14,8 @@
 // The barriers between the two CTAs use the default (CTA) scope: what they guard is read and written by the tensor cores and
 // the TMA engine, ordered by the proxy fence and the tensor-memory fences beside them.  With cluster-scope acquire in the
 // waits a k-block took 1.25 us instead of 0.66, whatever the depth of the rings.
-// Measured (kernel alone, one-CTA kernel in brackets): 11008 x 4096 at M = 4096 249 us = 1.48 PF/s (267), 5120 x 13696 400 us
-// (432), 4096 x 4096 at M = 2048 49.7 (53.1); at M = 999 on 13696 x 5120, 60 tiles of 384 tokens, 129 (144 to 158).
+// Measured (a call, one-CTA kernel in brackets): 11008 x 4096 at M = 4096 246 us = 1.50 PF/s (288), at M = 2048 125 (141),
+// 5120 x 13696 at M = 4096 400 (432), 4096 x 11008 at M = 2048 134 (147; 160 before its single threads were chosen by elect.sync).
 // Every wait is bounded (device status 2), tensor memory is freed on every path.
 #include "common.cuh"
 #include "kernels.h"
@@ -127,7 +127,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __re
 
     if (warp == 0) {
         // ------------------------------------------------------------------ activation producer
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0, d = 0, it = 0;      // d: slot of done[] for k-block it - NX
             uint32_t phd = 0;
             bool ok = true;
@@ -157,7 +157,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __re
     }
     else if (warp == 6) {
         // ------------------------------------------------------------------ int8 weight producer: this CTA's 128 channels
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0, it = 0;
             uint32_t ph = 1;
             bool ok = true;
@@ -188,7 +188,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __re
     }
     else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer of the pair
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             const uint32_t idesc = umma_idesc_f16(256, bn);
             const uint64_t b_desc0 = umma_desc_sw128(smem_u32(x_ring));
             const uint64_t a_desc0 = umma_desc_sw128(smem_u32(h_ring));

@@ -355,7 +355,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
 
     if (warp == 0) {
         // ------------------------------------------------------------------ activation producer
-        if (lane == 0) {
+        if (elect_one()) {
             // (ring positions are counters: this loop is one thread's chain of dependent instructions)
             int s = 0, d = 0, it = 0;      // d: slot of done[] for k-block it - NX
             uint32_t phd = 0;
@@ -384,7 +384,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
     }
     else if (warp == 6) {
         // ------------------------------------------------------------------ int8 weight producer
-        if (lane == 0) {
+        if (elect_one()) {
             int s = 0, it = 0;
             uint32_t ph = 1;
             bool ok = true;
@@ -414,7 +414,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
     }
     else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = umma_idesc_f16(128, bn);
             const uint64_t b_desc0 = umma_desc_sw128(smem_u32(x_ring));
             const uint64_t a_desc0 = umma_desc_sw128(smem_u32(h_ring));
