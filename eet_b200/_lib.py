@@ -26,6 +26,7 @@ SIGNATURES = {
     "eet_gemm_w8a16_workspace_bytes": (_sz, [_i, _i, _i]),
     "eet_gemm_w8a16": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _vp, _i, _vp, _sz, _vp]),
     "eet_gemm_w8a16_plan": (_i, [_i, _i, _i, _c.POINTER(_i)]),
+    "eet_gemm_w8a16_weights_in_tmem": (_i, [_i, _i, _i]),
     "eet_gemm_w8a16_row": (_i, [_vp, _vp, _vp, _f, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]),
     "eet_gemm_w8a16_noalloc": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _vp, _i, _vp]),
     "eet_gemm_w8a16_accum": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp]),

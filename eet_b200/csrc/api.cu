@@ -50,6 +50,7 @@ static inline bool aligned16(const void* p)
 #include "gemm_tc.cu"
 #include "gemm_mid.cu"
 #include "gemm_pair.cu"
+#include "gemm_ts.cu"
 #include "attention_tc.cu"
 #include "glue.cu"
 #include "noalloc.cu"
@@ -205,22 +206,31 @@ int eet_gemm_w8a16_finalize(float* sums, const void* scale, const void* residual
     return launch_finalize(sums, (const __half*)scale, (const __half*)residual, (__half*)C, M, N, (cudaStream_t)stream);
 }
 
-// Which kernel a shape goes to.  Up to 16 rows the row kernel, or equal shares with a finishing launch.  Above that stream-K units into fp32 scratch with a finishing
-// launch, tiles on single CTAs or tiles on CTA pairs, both with the epilogue fused: the shortest modelled time decides, among
-// those that the shape may take.  Measured on both sides of the lines: 4096 x 4096, M = 128 units 15 us, tiles 18, and at M = 256
+// Which kernel a shape goes to.  Up to 16 rows the row kernel, or equal shares with a finishing launch.  Above that tiles with the
+// weights in tensor memory (N and K large enough to have been measured), stream-K units into fp32 scratch with a finishing
+// launch, tiles with the weights in shared memory or tiles on CTA pairs, all but the units with the epilogue fused: the shortest
+// modelled time decides, among those that the shape may take; up to 64 rows it is the first kind, where it takes the shape
+// (4096 x 12288, M = 64: 14.9 us, stream-K 20.2; 11008 x 4096, M = 32: 14.2 and 13.9).  Measured on both sides of the lines: 4096 x 4096, M = 128 units 15 us, tiles 18, and at M = 256
 // 21.7 and 20.2; 4096 x 32000, M = 384 units 148, tiles 100, pairs 94; 11008 x 4096, M = 4096 single CTAs 267, pairs 249.
 enum { kRouteShares = 0, kRouteRow = 1, kRouteStreamK = 2, kRouteTiles = 3, kRoutePairs = 4 };
 
 struct GemmRoute {
     int kernel;
     bool sums;        // sums in the scratch, finished by another launch, are a way for this shape, chosen or not
+    bool ts;          // tiles: with the weights as an operand in tensor memory
     Tc2Plan tc;
     PairPlan pair;
 };
 
+// Above 64 rows the tiles with the weights in tensor memory must be modelled this much shorter than the best of the others, whose
+// models are off by 6 to 8 %: nearer than that the measured times were equal or the other way round (5120 x 13696, M = 1024:
+// modelled 106 us, measured 120, tiles with the weights in shared memory 114).  Stream-K has become a tenth faster than its
+// model since that was fitted (4096 x 4096, M = 100: 12.3 us, modelled 13.9, these tiles 11.2; M = 160: 17.2 and 12.6).
+constexpr double kTsMargin = 0.85, kTsMarginStreamK = 0.78;
+
 static GemmRoute gemm_route(int M, int N, int K, bool scratch)
 {
-    GemmRoute r = {kRouteShares, true, Tc2Plan{0, 0, 0, 1, 1e30}, PairPlan{0, 1e30}};
+    GemmRoute r = {kRouteShares, true, false, Tc2Plan{0, 0, 0, 1, 1e30}, PairPlan{0, 1e30}};
     if (M <= kRowMaxM) {
         if (!gemm_row_wastes_a_wave(M, N, K)) r.kernel = kRouteRow;
         return r;
@@ -236,7 +246,16 @@ static GemmRoute gemm_route(int M, int N, int K, bool scratch)
         r.kernel = kRouteTiles;
         least = r.tc.us;
     }
-    if (r.pair.us < least) r.kernel = kRoutePairs;
+    if (r.pair.us < least) {
+        r.kernel = kRoutePairs;
+        least = r.pair.us;
+    }
+    const Tc2Plan ts = gemm_ts_plan(M, N, K);
+    if (ts.us < (M < kTcMinM ? 1e30 : (r.kernel == kRouteStreamK ? kTsMarginStreamK : kTsMargin) * least)) {
+        r.kernel = kRouteTiles;
+        r.ts = true;
+        r.tc = ts;
+    }
     r.sums = r.sums || r.kernel == kRouteShares;
     return r;
 }
@@ -252,6 +271,12 @@ int eet_gemm_w8a16_plan(int M, int N, int K, int* plan)
     plan[3] = r.kernel == kRouteTiles ? r.tc.tiles - r.tc.whole : 0;
     plan[4] = r.kernel == kRouteTiles ? r.tc.split : 0;
     return 0;
+}
+
+int eet_gemm_w8a16_weights_in_tmem(int M, int N, int K)
+{
+    if (M <= 0 || N <= 0 || K <= 0 || K % 64 != 0 || N % 64 != 0) return 0;
+    return gemm_route(M, N, K, true).ts ? 1 : 0;
 }
 
 int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* C, int M, int N, int K,
@@ -270,8 +295,8 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
     // C over A: only sums that are finished by another launch let all of A be read before C is stored
     const uintptr_t a0 = (uintptr_t)A, a1 = a0 + (size_t)M * K * 2, c0 = (uintptr_t)C, c1 = c0 + (size_t)M * N * 2;
     if (route.sums && a0 < c1 && c0 < a1) route.kernel = gemm_mid_supported(M, N, K) ? kRouteStreamK : kRouteShares;
-    // (up to 16 rows this entry point has always asked for it, whichever kernel serves)
-    EET_CHECK(scratch || (M > kRowMaxM && route.kernel != kRouteStreamK && route.kernel != kRouteShares),
+    // (up to 64 rows this entry point has always asked for it, whichever kernel serves)
+    EET_CHECK(scratch || (M >= kTcMinM && route.kernel != kRouteStreamK && route.kernel != kRouteShares),
               "eet_gemm_w8a16: workspace of %zu bytes is smaller than the %zu needed", ws_bytes,
               eet_gemm_w8a16_workspace_bytes(M, N, K));
     if (route.kernel == kRouteRow) {
@@ -291,6 +316,10 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
     if (route.kernel == kRoutePairs) {
         return launch_gemm_pair((const __half*)A, (const uint8_t*)packedB, (const __half*)scale, (__half*)C, res, gate, M, N, K,
                                 route.pair.bn, (cudaStream_t)stream);
+    }
+    if (route.kernel == kRouteTiles && route.ts) {
+        return launch_gemm_ts((const __half*)A, (const uint8_t*)packedB, (const __half*)scale, (__half*)C, res, gate, M, N, K,
+                              route.tc, (cudaStream_t)stream);
     }
     if (route.kernel == kRouteTiles) {
         return launch_gemm_tc((const __half*)A, (const uint8_t*)packedB, (const __half*)scale, (__half*)C, res, gate, M, N, K,

@@ -71,7 +71,8 @@ struct MidSmem {
     volatile int abort;
 };
 
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32])
+// (the caller waits for the stores before it tells anybody)
+__device__ __forceinline__ void tmem_st32_async(uint32_t taddr, const uint32_t (&v)[32])
 {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -82,6 +83,11 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
         "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
         "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
         : "memory");
+}
+
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32])
+{
+    tmem_st32_async(taddr, v);
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 

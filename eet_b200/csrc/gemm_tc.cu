@@ -20,9 +20,8 @@
 //  Every wait is bounded; a wait that runs out sets the device status word, and the CTA still frees its
 //  tensor memory before it returns.
 //
-// Measured and not taken: the fp16 weights in tensor memory as the MMA's A operand (BN up to 192 beside the accumulators,
-// one or two sets of eight conversion warps, two to four buffers): 0.78 us a k-block at BN = 192 and 0.65 at 128, against
-// 0.69 and 0.62 here; moving the bytes alone takes 0.41, i.e. 98 B/ns an SM from L2.
+// (The weights in tensor memory as the MMA's A operand: gemm_ts.cu, which takes most shapes whose tiles fill a wave or less.  Here a
+// k-block is bound by shared memory, 768 + 3 BN cycles, and by the 98 B/ns that an SM gets from L2.)
 //
 // Numerics: exact integer weights as fp16, fp32 accumulation, one multiply by the fp16 scale, one rounding
 // to fp16 - the same as the skinny kernel's finalize step.
@@ -236,6 +235,7 @@ static_assert(kTc2StageBytes <= kTc2NH * 2 * kTc2HBytes, "stream-K mode stages i
 
 // Barrier of the 256 transform/epilogue threads of the 256 x 256 kernel that also ORs a predicate over them:
 // every thread gets the same answer, so a decision taken on it cannot split the group before a later barrier.
+template<int kThreads = 256>
 __device__ __forceinline__ bool epi_bar_or(bool pred)
 {
     uint32_t out;
@@ -243,11 +243,11 @@ __device__ __forceinline__ bool epi_bar_or(bool pred)
         "{\n\t"
         ".reg .pred p, q;\n\t"
         "setp.ne.u32 q, %1, 0;\n\t"
-        "bar.red.or.pred p, 3, 256, q;\n\t"
+        "bar.red.or.pred p, 3, %2, q;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t"
         "}\n"
         : "=r"(out)
-        : "r"((uint32_t)pred)
+        : "r"((uint32_t)pred), "n"(kThreads)
         : "memory");
     return out != 0;
 }

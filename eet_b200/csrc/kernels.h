@@ -62,6 +62,12 @@ Tc2Plan gemm_tc_plan(int M, int N, int K);
 int launch_gemm_tc(const __half* A, const uint8_t* B, const __half* scale, __half* C, const __half* residual, int gate,
                    int M, int N, int K, const Tc2Plan& plan, cudaStream_t stream);
 
+// gemm_ts.cu (tcgen05, the weights as an operand in tensor memory)
+constexpr int kTsMinM = 17, kTsMinN = 4096, kTsMinK = 2048;
+Tc2Plan gemm_ts_plan(int M, int N, int K);   // `whole` or the others, not both
+int launch_gemm_ts(const __half* A, const uint8_t* B, const __half* scale, __half* C, const __half* residual, int gate,
+                   int M, int N, int K, const Tc2Plan& plan, cudaStream_t stream);
+
 // gemm_pair.cu (tcgen05 on CTA pairs)
 struct PairPlan {
     int bn;       // tokens per accumulator; 0: the kernel does not take the shape

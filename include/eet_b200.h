@@ -109,10 +109,11 @@ size_t eet_gemm_w8a16_workspace_bytes(int M, int N, int K);
  * M may be any value >= 0; K and N must be multiples of 64; pointers 16-byte aligned.  C may lie over A up to 64 rows, and up
  * to 512 for narrow shapes (below), with scratch.
  * Kernels: M <= 16 the row kernel (one launch, leaves the scratch alone), wide matrices that would leave its last wave
- * mostly empty the equal-share kernel into the scratch with a finishing launch; 16 < M <= 64 (N % 128 == 0) stream-K
- * into the scratch with a finishing launch; above that the shortest of three modelled times decides between stream-K (up
- * to 512 rows), tiles of 256 channels on single CTAs or with the reduction split over clusters of 2-4, and tiles on CTA
- * pairs (from 256 rows); shapes with N % 128 == 64 take the equal-share kernel in groups of 128 rows.
+ * mostly empty the equal-share kernel into the scratch with a finishing launch; 16 < M <= 64 (N % 128 == 0) tiles of 256
+ * channels with the weights in tensor memory (N >= 4096, K >= 2048) or stream-K into the scratch with a finishing launch;
+ * above that the shortest modelled time decides between these, tiles with the weights in shared memory, both on single CTAs
+ * or with the reduction split over clusters of 2-8, and tiles on CTA pairs (from 256 rows); shapes with N % 128 == 64 take
+ * the equal-share kernel in groups of 128 rows.
  * Scratch is needed for M <= 64, for N % 128 == 64, and for C over A.  Up to 512 rows, narrow shapes (N % 256 != 0, or
  * 256 x 256 tiles so few that not 96 CTAs, or 120 without a split, would share them) use it where that is faster and go
  * to tiles without it; the others always go to tiles.  Tiles and the row kernel give the same bits every time, stream-K
@@ -124,11 +125,14 @@ int eet_gemm_w8a16(const void* A, const void* packedB, const void* scale, void* 
 /*
  * The kernel that eet_gemm_w8a16 gives a shape to on the current device, for tests and tools; launches nothing.
  *   plan[0]  0 equal shares into the scratch (gemm_skinny.cu), 1 row kernel (gemm_row.cu), 2 stream-K into the scratch
- *            (gemm_mid.cu), 3 tiles on single CTAs or clusters (gemm_tc.cu), 4 tiles on CTA pairs (gemm_pair.cu)
+ *            (gemm_mid.cu), 3 tiles on single CTAs or clusters (gemm_ts.cu, gemm_tc.cu), 4 tiles on CTA pairs (gemm_pair.cu)
  *   plan[1]  tokens per tile (3 and 4)
  *   plan[2], plan[3], plan[4]  with 3: tiles on single CTAs, tiles whose reduction is split over a cluster, its size
  */
 int eet_gemm_w8a16_plan(int M, int N, int K, int* plan);
+
+/* 1 if those are tiles with the weights as an operand in tensor memory (gemm_ts.cu), else 0; for tests and tools. */
+int eet_gemm_w8a16_weights_in_tmem(int M, int N, int K);
 
 /*
  * The decode GEMM (M <= 16) with what stands around it in a decoder layer, in one launch and without scratch:

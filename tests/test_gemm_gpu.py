@@ -247,6 +247,56 @@ def test_prefill_gemm_tiles(K, N, M, kernel, whole, split, kind):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("K,N,M,bn,split,tiles", [
+    (2112, 22016, 17, 32, 1, 86), (2112, 11008, 17, 32, 3, 43), (2112, 4096, 17, 32, 6, 16), (4096, 8320, 33, 48, 4, 33),
+    (2112, 4096, 161, 48, 2, 64), (4096, 5120, 50, 64, 5, 20), (2112, 5120, 111, 64, 3, 40), (2112, 4096, 129, 80, 4, 32),
+    (4096, 22016, 233, 80, 1, 258), (2112, 8320, 90, 96, 4, 33), (11008, 5120, 100, 112, 6, 20), (2112, 22016, 300, 112, 1, 258),
+    (4096, 4096, 233, 128, 4, 32), (4096, 12288, 127, 128, 2, 48), (2112, 22016, 385, 144, 1, 258), (5120, 4352, 150, 160, 6, 17),
+    (2112, 8320, 700, 176, 1, 132), (11008, 5120, 333, 176, 3, 40), (11008, 5120, 190, 192, 6, 20), (2112, 22016, 190, 192, 1, 86)])
+@pytest.mark.parametrize("kind", ["plain", "residual", "gate"])
+def test_tiles_with_the_weights_in_tensor_memory(K, N, M, bn, split, tiles, kind):
+    """Every token tile from the smallest to the largest, units of one and of two k-blocks and an odd k-block at the end (K =
+    2112), clusters of every size that a plan uses, chunks of 8 and of 16 tokens with fewer chunks than ranks, persistent CTAs
+    with several tiles, a last channel tile of half height (N = 8320); the plan is part of the case.  Bound: one fp16 rounding
+    of the product and one of the sum, 2^-11 each, doubled; the activation's error is its operands' plus its own fp16 steps.
+    And the same bits from a second call behind a call on other rows."""
+    from eet_b200 import EET, _lib
+    assert _lib.lib.eet_gemm_w8a16_weights_in_tmem(M, N, K) == 1
+    assert _plan(M, N, K) == (TILES, bn, tiles if split == 1 else 0, 0 if split == 1 else tiles, split)
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    q = torch.randint(-127, 128, (K, N), generator=gen, device="cuda", dtype=torch.int8)
+    s = ((torch.rand(N, generator=gen, device="cuda") + 0.5) * K ** -0.5 / 64).half()
+    x = torch.randn(M, K, generator=gen, device="cuda").half()
+    other = torch.randn(M, N, generator=gen, device="cuda").half()
+    packed = EET.preprocess_weights(q)
+    out = torch.full((M + 1, N), 7.0, dtype=torch.float16, device="cuda")
+    kw = {"residual": {"residual": other}, "gate": {"gate": other}}.get(kind, {})
+    EET.gemm_w8a16(x, packed, s, out=out[:M], **kw)
+    EET.gemm_w8a16(x.flip(0), packed, s, **kw)
+    again = EET.gemm_w8a16(x, packed, s, **kw)
+    y = (x.double() @ q.double()) * s.double()
+    if kind == "gate":
+        want = torch.nn.functional.silu(other.double()) * y
+        tol = 2.0 ** -10 * (4 * want.abs() + y.abs()) + 1e-4
+    else:
+        want = y + (other.double() if kind == "residual" else 0)
+        tol = 2.0 ** -10 * (y.abs() + want.abs()) + 1e-4
+    assert ((out[:M].double() - want).abs() <= tol).all()
+    assert torch.equal(out[:M], again) and bool((out[M] == 7.0).all())
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("K,N,M,taken", [
+    (4096, 4096, 16, 0), (4096, 4096, 17, 1), (4096, 3968, 40, 0), (1984, 4096, 40, 0), (4096, 4224, 40, 0), (4096, 8320, 40, 1),
+    (4096, 4096, 64, 1), (4096, 4096, 100, 0), (4096, 11008, 100, 1), (13696, 5120, 999, 1), (5120, 13696, 999, 0), (4096, 4096, 4096, 0)])
+def test_shapes_that_go_to_tensor_memory(K, N, M, taken):
+    """Both sides of each line of the rule; and up to 64 rows the entry point still refuses a call without scratch."""
+    from eet_b200 import _lib
+    assert _lib.lib.eet_gemm_w8a16_weights_in_tmem(M, N, K) == taken
+    if M <= 64:
+        assert _lib.lib.eet_gemm_w8a16(16, 16, 16, 16, M, N, K, None, 0, None, 0, None) != 0 and b"workspace" in _lib.lib.eet_last_error()
+
+
 @pytest.mark.parametrize("kind", ["plain", "residual", "gate", "gated", "norm", "norm_gated"])
 @pytest.mark.parametrize("K,N,M", [(64, 64, 1), (512, 128, 16), (1088, 64, 9), (1088, 2560, 8), (4096, 4096, 7), (5120, 5120, 3),
                                    (2048, 8192, 13), (5120, 13696, 12), (64, 65536, 2)])
