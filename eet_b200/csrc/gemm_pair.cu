@@ -390,7 +390,9 @@ PairPlan gemm_pair_plan(int M, int N, int K)
     for (int bn = 256; bn >= 128; bn -= 16) {
         const long long tiles = (long long)tiles_n * ((M + 2 * bn - 1) / (2 * bn));
         if (tiles > 0x3fffffffLL) continue;
-        const double block = 0.65 + 0.00203 * (bn - 192);   // a k-block with the machine full, measured at BN = 192 and 256
+        // a k-block with the machine full: fitted to 110 calls of 256 to 4096 rows at K from 4096 on; below, where a tile's start and
+        // end weigh as much, as measured before its threads were chosen by elect.sync
+        const double block = K >= 4096 ? 0.60 + 0.0018 * (bn - 192) : 0.65 + 0.00203 * (bn - 192);
         const double us = 7.0 + (double)((tiles + pairs - 1) / pairs) * (KT * block + 1.5 + 0.01 * bn);
         if (us < best.us) best = PairPlan{bn, us};
     }

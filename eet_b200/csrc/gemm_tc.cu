@@ -355,7 +355,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
 
     if (warp == 0) {
         // ------------------------------------------------------------------ activation producer
-        if (elect_one()) {
+        // (lane 0 and not elect.sync, here and for the weights: producers that run further ahead take the CTAs of a wave out of
+        // step - 22016 x 8192 at M = 1426: 463 us, 448 so)
+        if (lane == 0) {
             // (ring positions are counters: this loop is one thread's chain of dependent instructions)
             int s = 0, d = 0, it = 0;      // d: slot of done[] for k-block it - NX
             uint32_t phd = 0;
@@ -384,7 +386,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t* __res
     }
     else if (warp == 6) {
         // ------------------------------------------------------------------ int8 weight producer
-        if (elect_one()) {
+        if (lane == 0) {
             int s = 0, it = 0;
             uint32_t ph = 1;
             bool ok = true;
