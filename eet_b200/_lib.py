@@ -40,6 +40,7 @@ SIGNATURES = {
     "eet_qkv_split_store": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _vp]),
     "eet_prefill_mha": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp, _i, _vp]),
     "eet_decode_mha": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _i, _vp, _i, _f, _i, _vp]),
+    "eet_mmha_decode": (_i, [_vp, _vp, _f] + [_vp] * 10 + [_i] * 6 + [_vp, _vp, _i, _i, _f, _vp, _sz, _vp]),
     "eet_decode_mha_plan": (_i, [_i, _i, _i, _c.POINTER(_i)]),
     "eet_reorder_kv_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "eet_reorder_kv": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _sz, _vp]),

@@ -514,6 +514,26 @@ int eet_decode_mha(const void* qkv, float* qkv_sums, const void* qkv_scale, void
     return launch_decode_mha(a, (cudaStream_t)stream);
 }
 
+int eet_mmha_decode(const void* x, const void* gamma, float eps, void* xn, const void* qkv_w, const void* qkv_scale, void* qkv,
+                    void* kcache, void* vcache, void* ctx, const void* out_w, const void* out_scale, void* out, int B, int H,
+                    int D, int T_max, int hidden, int step, const int64_t* pad_len, const void* alibi, int alibi_stride, int rope,
+                    float rope_base, void* ws, size_t ws_bytes, void* stream)
+{
+    const int inner = H * D;
+    auto linear = [&](const void* a, const void* w, const void* scale, void* c, int n, int k, const void* residual) {
+        // (without scratch only the row kernel, which the caller has made sure serves this width)
+        if (B <= kRowMaxM && ws == nullptr) {
+            return eet_gemm_w8a16_row(a, nullptr, nullptr, 0.f, w, scale, nullptr, nullptr, residual, c, nullptr, B, n, k, stream);
+        }
+        return eet_gemm_w8a16(a, w, scale, c, B, n, k, residual, residual != nullptr ? 1 : 0, ws, ws_bytes, stream);
+    };
+    if (int rc = eet_rmsnorm(x, gamma, xn, B, hidden, eps, stream)) return rc;
+    if (int rc = linear(xn, qkv_w, qkv_scale, qkv, 3 * inner, hidden, nullptr)) return rc;
+    if (int rc = eet_decode_mha(qkv, nullptr, qkv_scale, kcache, vcache, ctx, B, H, D, T_max, step, nullptr, pad_len, alibi,
+                                alibi_stride, nullptr, rope, rope_base, 0, stream)) return rc;
+    return linear(ctx, out_w, out_scale, out, hidden, inner, x);
+}
+
 size_t eet_reorder_kv_workspace_bytes(int B, int H, int D, int step)
 {
     return (size_t)2 * B * H * step * D * sizeof(__half);

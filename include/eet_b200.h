@@ -272,6 +272,20 @@ int eet_decode_mha(const void* qkv, float* qkv_sums, const void* qkv_scale, void
                    const void* alibi, int alibi_stride, const float* alibi_slopes, int rope, float rope_base, int splits,
                    void* stream);
 
+/*
+ * One decode step of an attention block in one call: rmsnorm(x) -> xn, QKV projection -> qkv, decode attention -> ctx, output
+ * projection + x -> out; the launches of eet_rmsnorm, eet_gemm_w8a16 (up to 16 rows without scratch eet_gemm_w8a16_row),
+ * eet_decode_mha and again the projection, in this order, with their checks.
+ * Replaces: LlamaMmha::forward_inc / BaichuanMmha::forward_inc (csrc/op/llama_mmha.cpp:204-266).
+ *   x, xn, out [B][hidden]; qkv [B][3][H][D]; ctx [B][H*D]; weights W8T64 [hidden][3*H*D] and [H*D][hidden] with their scales
+ *   step, pad_len, alibi, alibi_stride, rope, rope_base   as in eet_decode_mha
+ *   ws   scratch of eet_gemm_w8a16 for the wider projection; NULL up to 16 rows: then both go to the row kernel
+ */
+int eet_mmha_decode(const void* x, const void* gamma, float eps, void* xn, const void* qkv_w, const void* qkv_scale, void* qkv,
+                    void* kcache, void* vcache, void* ctx, const void* out_w, const void* out_scale, void* out, int B, int H,
+                    int D, int T_max, int hidden, int step, const int64_t* pad_len, const void* alibi, int alibi_stride, int rope,
+                    float rope_base, void* ws, size_t ws_bytes, void* stream);
+
 /* What splits = 0 chooses on the current device for histories of up to `len` steps, for tests and tools; launches nothing:
  * plan[0] CTAs per (batch, head), plan[1] CTAs per SM that the kernel is built for (4 or 5). */
 int eet_decode_mha_plan(int B, int H, int len, int* plan);

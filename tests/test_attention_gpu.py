@@ -292,3 +292,47 @@ def test_decode_finishes_projection_sums_itself():
     assert _close(ctx.cpu().view(B, H, D), ref)
     assert _close(kc.cpu()[:, :, step - 1], kc_ref[:, :, step - 1])
     assert float(sums_c.abs().max()) == 0
+
+
+@pytest.mark.parametrize("B,heads,alibi,pad", [(1, 2, False, False), (3, 2, False, True), (16, 32, False, False), (16, 40, True, False),
+                                               (17, 2, True, False), (40, 32, False, True), (8, 64, False, False)])
+def test_decode_op_alone_is_the_chain_of_its_kernels(B, heads, alibi, pad):
+    """The op's call of its own (one call into the library) against the kernels called one by one, three steps: 64 heads are wide
+    enough for scratch below 16 rows, 17 and 40 rows need it.  Same kernels, same order; only sums that meet in the order of
+    arrival (2 heads, 17 rows; 64 heads) may round the last bit of a projection differently."""
+    from eet_b200 import EET
+    from eet_b200._lib import check, lib
+    h, D, T, hist = heads * 128, 128, 80, 37
+    gen = torch.Generator(device="cuda").manual_seed(B)
+
+    def mat(K, N):
+        return (EET.preprocess_weights(torch.randint(-127, 128, (K, N), generator=gen, device="cuda", dtype=torch.int8)),
+                ((torch.rand(N, generator=gen, device="cuda") + 0.5) * K ** -0.5 / 64).half())
+
+    (w0, s0), (w1, s1) = mat(h, 3 * h), mat(h, h)
+    ln = (1 + 0.1 * torch.randn(h, generator=gen, device="cuda")).half()
+    none = torch.empty(0)
+    desc = EET.MetaDesc(torch.float16, B, heads, h, 1, hist, T, "silu", D, 4 * h, "cuda:0", False, 1e-6, True)
+    op = (EET.BaichuanMmha if alibi else EET.LlamaMmha)(desc, w0, s0, none, none, none, w1, s1, none, ln, none)
+    op.k_cache[:, :, :hist] = torch.randn(B, heads, hist, D, generator=gen, device="cuda").half()
+    op.v_cache[:, :, :hist] = torch.randn(B, heads, hist, D, generator=gen, device="cuda").half()
+    kc, vc = op.k_cache.clone(), op.v_cache.clone()
+    op.step_ = hist
+    pads = (torch.arange(B, device="cuda") % 7).view(B, 1) if pad else none
+    for step in range(hist + 1, hist + 4):
+        x = torch.randn(B, 1, h, generator=gen, device="cuda").half()
+        bias = ops.alibi_mask(heads, T).half()[:, step - 1: step, :step].contiguous().cuda() if alibi else none
+        got = op.forward(x, pads, none, True, True, False, bias).clone()
+        xn = torch.empty(B, h, dtype=torch.float16, device="cuda")
+        check(lib.eet_rmsnorm(x.data_ptr(), ln.data_ptr(), xn.data_ptr(), B, h, 1e-6, _stream()))
+        qkv = EET.gemm_w8a16(xn, w0, s0).view(B, 3, heads, D)
+        ctx = torch.empty(B, h, dtype=torch.float16, device="cuda")
+        check(lib.eet_decode_mha(qkv.data_ptr(), None, None, kc.data_ptr(), vc.data_ptr(), ctx.data_ptr(), B, heads, D, T, step, None,
+                                 pads.data_ptr() if pad else None, bias.data_ptr() if alibi else None, step if alibi else 0, None,
+                                 0 if alibi else 1, 10000.0, 0, _stream()))
+        want = EET.gemm_w8a16(ctx, w1, s1, residual=x.view(B, h)).view(B, 1, h)
+        if (B > 16 and heads == 2) or heads == 64:
+            assert _close(got, want) and _close(op.k_cache, kc) and _close(op.v_cache, vc)
+        else:
+            assert torch.equal(got, want) and torch.equal(op.k_cache, kc) and torch.equal(op.v_cache, vc)
+    assert op.step_ == hist + 3
