@@ -38,7 +38,7 @@ void set_error(const char* fmt, ...);
 // Device-side status word.  A kernel that had to give up stores a non-zero code here and returns normally (uniform
 // control flow, tensor memory freed, nothing left in flight); the host reads and clears it with eet_device_status().
 //   1  decode GEMM (gemm_skinny): a shared-memory pipeline wait ran out
-//   2  tensor-core GEMMs (gemm_mid, gemm_tc): a pipeline or tensor-memory wait ran out
+//   2  tensor-core GEMMs (gemm_ts, gemm_mid, gemm_tc, gemm_pair) and prefill attention: a pipeline or tensor-memory wait ran out
 //   3  decode attention: a pipeline wait ran out
 //   4  tensor-parallel exchange: a peer's partial sums never arrived in this rank's inbox
 //   5  decode attention: the device-resident step was outside [1, cache length]; nothing was appended
