@@ -361,8 +361,8 @@ def cpu_decode_sample(steps, warmup=1, budget_s=15.0, threads=None):
 
 def profile_kernels():
     """A handful of launches for profiler captures (`--profile-kernels`): the quantizer on K=4096, N=11008, the row kernel at
-    M = 8 on K=4096, N=12288, the stream-K kernel at M = 32 on K=8192, N=22016 and at M = 100 on K=N=4096, the tile kernel
-    at M = 1024 on K=11008, N=4096 (split-K over clusters of two), CTA pairs at M = 4096 on the same; three more GEMMs of
+    M = 8 on K=4096, N=12288, tiles with the weights in tensor memory at M = 32 on K=8192, N=22016, the stream-K kernel at
+    M = 100 on K=N=4096, the tile kernel at M = 1024 on K=11008, N=4096 (split-K over clusters of two), CTA pairs at M = 4096 on the same; three more GEMMs of
     earlier captures; and the prefill attention at B=8, H=32, S=512.  Each launch of a GEMM gets weights of its own; nothing
     is timed or printed but the device status."""
     from eet_b200 import EET, _lib
