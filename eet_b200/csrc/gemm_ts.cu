@@ -23,7 +23,7 @@
 // 13696 x 5120 at M = 1024: 107 (152).
 // Not taken: three sets of conversion warps (instruction issue is what they share: 850 cycles a k-block); one set and two CTAs per SM
 // (4096 x 11008, M = 32: 14.9 us, 13.0 here); partial sums through the copy engine (16.9 us at M = 100, 16.5 as they are).
-// Every wait is bounded (device status 2) and tensor memory is freed on every path.
+// Every wait is bounded (device status 2), tensor memory is freed on every path, and the CTAs of a cluster end together.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -107,6 +107,18 @@ __device__ __forceinline__ uint32_t cluster_addr32(uint32_t local, int rank)
 }
 __device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank) { return cluster_addr32(smem_u32(p), rank); }
 
+// This warp's part of a cluster-wide barrier; the CTAs of the cluster are past it when cluster_wait returns.
+__device__ __forceinline__ void cluster_arrive()
+{
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait()
+{
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ void prefetch_map(const CUtensorMap* map)
 {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
@@ -162,16 +174,21 @@ template<>
 __device__ __forceinline__ void tmem_ld_tokens<16>(uint32_t taddr, uint32_t (&v)[16]) { tmem_ld16(taddr, v); }
 
 // The S partial accumulators of a cluster meet through distributed shared memory.  The tile's tokens are dealt out to the ranks in
-// chunks of T (chunk q belongs to rank q % S).  A CTA whose MMAs have completed has told the others that its rings may be
-// overwritten; each stores its partials of foreign chunks into their owners' and, once all bytes of its own chunks have
-// arrived, adds them to its own sums in rank order and finishes its chunks.
+// chunks of T (chunk q belongs to rank q % S).  A CTA whose MMAs have completed (`summed`) has told the others that its rings may
+// be overwritten; each stores its partials of foreign chunks into their owners' and, once all bytes of its own chunks have
+// arrived, adds them to its own sums in rank order and finishes its chunks.  A CTA whose wait for its MMAs or for the others ran
+// out stores nothing into anybody; who waits for its partials gives up in turn.  Behind its last store every thread arrives at
+// the cluster barrier, which the kernel waits for before it ends: no CTA leaves while another may still address it.
 template<int T>
 __device__ __forceinline__ void ts_exchange(TsSmem& sm, const TsArgs& a, uint8_t* base, uint8_t* stage_base, uint32_t tmem, float sc, int warp,
-                                            int lane, int S, int rank, int n0, int m0)
+                                            int lane, int S, int rank, int n0, int m0, bool summed)
 {
     constexpr int kBytes = 256 * T * 4;   // the partial sums of a chunk
     const int set = (warp - 3) >> 3, grp = ((warp - 3) >> 2) & 1;
-    if (warp < 3 || (grp == 1 && n0 + 128 >= a.N)) return;   // (the last tile may have no upper half)
+    if (warp < 3 || (grp == 1 && n0 + 128 >= a.N)) {   // (the last tile may have no upper half)
+        cluster_arrive();
+        return;
+    }
     const int tw = ((warp - 3) & 3) * 32 + lane, lane_base = (warp & 3) * 32, r = lane_base + lane;
     const int chunks = (min(a.M, m0 + a.bn) - m0 + T - 1) / T;
     const uint32_t acc = tmem + ((uint32_t)lane_base << 16) + (uint32_t)(grp * a.acc_cols);
@@ -189,11 +206,11 @@ __device__ __forceinline__ void ts_exchange(TsSmem& sm, const TsArgs& a, uint8_t
         }
     };
     fetch(rank + S * set);
-    tc_wait_warp(&sm.peers_done, 0, &sm.abort);
+    const bool send = tc_wait_warp(&sm.peers_done, 0, &sm.abort) && summed;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t local = smem_u32(base) + mine, bar_local = smem_u32(&sm.partials);
     int owner = set, turn = 0;   // chunk q = turn * S + owner
-    for (int q = set; q < chunks; q += kTsSets, owner += kTsSets) {
+    for (int q = set; q < chunks && send; q += kTsSets, owner += kTsSets) {
         while (owner >= S) {
             owner -= S;
             ++turn;
@@ -211,6 +228,7 @@ __device__ __forceinline__ void ts_exchange(TsSmem& sm, const TsArgs& a, uint8_t
                          : "memory");
         }
     }
+    cluster_arrive();
     // the partials of this CTA's chunks have arrived
     if (rank < chunks) tc_wait_warp(&sm.partials, 0, &sm.abort);
     __half* stage = reinterpret_cast<__half*>(stage_base) + (set * 2 + grp) * kTsStageHalves;
@@ -312,10 +330,11 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // waited for before the first remote access
+    if (S > 1) cluster_arrive();   // waited for before the first remote access
     const uint32_t tmem = sm.tmem_base;
     const uint32_t a_cols = tmem + 2 * (uint32_t)a.acc_cols;   // the fp16 weights: [buffer][half of the channels][32 columns]
     float sc = 0.f;          // conversion warps: the scale of this thread's channel
+    bool summed = false;     // and whether all MMAs of the last tile have completed, the same for a warp
 
     if (warp == 0) {
         // ------------------------------------------------------------------ activation producer
@@ -493,7 +512,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             // ---- end of the tile: every epilogue warp gets here, also one that has left the loop above because a wait ran out
             // (the others may have finished theirs); the OR-reducing barrier gives all epilogue threads the same answer, whoever
             // saw the abort flag first ----
-            if (ok) tc_wait_warp(&sm.accum, (uint32_t)(p & 1), &sm.abort);
+            summed = ok && tc_wait_warp(&sm.accum, (uint32_t)(p & 1), &sm.abort);
             if (S > 1) break;   // the exchange and the epilogue follow below, whatever ran out
             if (epi_bar_or<256 * kTsSets>(sm.abort != 0)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -516,11 +535,12 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     }
 
     if (S > 1) {
-        __syncwarp();
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // (long since complete: all have started)
-        if (warp == 3 && lane < S && lane != rank) mbar_arrive_cluster(cluster_addr(&sm.peers_done, lane));
-        if (ts_chunk(a.bn) == 8) ts_exchange<8>(sm, a, base, stage_base, tmem, sc, warp, lane, S, rank, (first / tiles_m) * 256, (first % tiles_m) * a.bn);
-        else ts_exchange<16>(sm, a, base, stage_base, tmem, sc, warp, lane, S, rank, (first / tiles_m) * 256, (first % tiles_m) * a.bn);
+        cluster_wait();   // (long since complete: all have started)
+        if (warp == 3 && summed && lane < S && lane != rank) mbar_arrive_cluster(cluster_addr(&sm.peers_done, lane));
+        const int n0 = (first / tiles_m) * 256, m0 = (first % tiles_m) * a.bn;
+        if (ts_chunk(a.bn) == 8) ts_exchange<8>(sm, a, base, stage_base, tmem, sc, warp, lane, S, rank, n0, m0, summed);
+        else ts_exchange<16>(sm, a, base, stage_base, tmem, sc, warp, lane, S, rank, n0, m0, summed);
+        cluster_wait();   // nobody will address this CTA's memory any more
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -47,3 +47,44 @@ def test_no_store_into_another_cta_before_it_is_known_to_run(name, push):
     text = _source(name)
     before = text[:text.index(push)]
     assert "barrier.cluster.wait" in before or "this_cluster().sync()" in before
+
+
+def _body(text, head):
+    """The braces behind `head`, and what they hold."""
+    start = text.index("{", text.index(head))
+    depth = 0
+    for i in range(start, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[start:i + 1]
+    raise AssertionError(head)
+
+
+@pytest.mark.parametrize("name,remote", [("gemm_tc.cu", "st.shared::cluster"), ("gemm_pair.cu", "mbar_arrive_cluster("),
+                                         ("gemm_ts.cu", "ts_exchange<")])
+def test_no_cta_leaves_while_another_of_its_cluster_may_address_it(name, remote):
+    """Also where a wait has run out: between a kernel's last remote access and the release of its tensor memory stands a
+    barrier of the whole cluster, and nothing jumps over it."""
+    text = _source(name)
+    tail = text[text.rindex(remote):]
+    tail = tail[:tail.index("tcgen05.dealloc")]
+    assert re.search(r"this_cluster\(\)\.sync\(\)|\bcluster_wait\(\)", tail)
+    assert not re.search(r"\b(return|goto)\b", tail)
+
+
+def test_exchange_arrives_at_the_cluster_barrier_once_behind_its_last_store():
+    """gemm_ts: every way through the exchange arrives once - before it waits for what the others send, behind its own stores -
+    and only a CTA whose MMAs have completed, and which knows that of the others, stores into them or lets them store."""
+    text = _source("gemm_ts.cu")
+    body = _body(text, "void ts_exchange(")
+    left = _body(body, "if (warp < 3 ||")
+    assert re.fullmatch(r"\{\s*cluster_arrive\(\);\s*return;\s*\}", left)
+    rest = body[body.index(left) + len(left):]
+    assert "return" not in rest and rest.count("cluster_arrive()") == 1
+    assert rest.rindex("st.async") < rest.index("cluster_arrive()") < rest.index("&sm.partials, 0")
+    stores = rest[:rest.index("cluster_arrive()")]
+    assert "send = tc_wait_warp(&sm.peers_done, 0, &sm.abort) && summed;" in stores
+    assert re.search(r"for \([^)]*&& send;", stores)
+    kernel = _body(text, "gemm_ts_kernel(")
+    assert "summed = ok && tc_wait_warp(&sm.accum" in kernel
+    assert re.search(r"if \([^)]*\bsummed\b.*\) mbar_arrive_cluster\(cluster_addr\(&sm.peers_done", kernel)
