@@ -206,8 +206,7 @@ def test_empty_and_invalid():
     packed = EET.preprocess_weights(q).cuda()
     out = EET.gemm_w8a16(torch.empty(0, 64, device="cuda").half(), packed, s.cuda())
     assert out.shape == (0, 64)
-    x, w = torch.zeros(1, 128, dtype=torch.float16, device="cuda"), torch.zeros(128, 64, dtype=torch.int8, device="cuda")
-    rc = _lib.lib.eet_gemm_w8a16(x.data_ptr(), w.data_ptr(), x.data_ptr(), x.data_ptr(), 1, 64, 100, None, 0, None, 0, None)
+    rc = _lib.lib.eet_gemm_w8a16(1, 1, 1, 1, 1, 64, 100, None, 0, None, 0, None)
     assert rc != 0
 
 
@@ -295,12 +294,7 @@ def test_shapes_that_go_to_tensor_memory(K, N, M, taken):
     from eet_b200 import _lib
     assert _lib.lib.eet_gemm_w8a16_weights_in_tmem(M, N, K) == taken
     if M <= 64:
-        x, out = torch.zeros(M, K, dtype=torch.float16, device="cuda"), torch.full((M, N), 7.0, dtype=torch.float16, device="cuda")
-        w, s = torch.zeros(K, N, dtype=torch.int8, device="cuda"), torch.zeros(N, dtype=torch.float16, device="cuda")
-        rc = _lib.lib.eet_gemm_w8a16(x.data_ptr(), w.data_ptr(), s.data_ptr(), out.data_ptr(), M, N, K, None, 0, None, 0,
-                                     torch.cuda.current_stream().cuda_stream)
-        assert rc != 0 and b"workspace" in _lib.lib.eet_last_error()
-        assert bool((out == 7.0).all())
+        assert _lib.lib.eet_gemm_w8a16(16, 16, 16, 16, M, N, K, None, 0, None, 0, None) != 0 and b"workspace" in _lib.lib.eet_last_error()
 
 
 @pytest.mark.parametrize("kind", ["plain", "residual", "gate", "gated", "norm", "norm_gated"])
