@@ -200,6 +200,21 @@ def test_repeated_calls_leave_scratch_clean(K, N, M):
     _check(y, x, q, s)
 
 
+@pytest.mark.parametrize("K,N,M", [(100, 64, 1), (128, 100, 1), (4096, 4096, 16), (4096, 4096, 17), (4096, 3968, 40), (1984, 4096, 40),
+                                   (4096, 8320, 40), (4096, 4096, 64)])
+def test_a_refused_call_stores_nothing(K, N, M):
+    """Sizes that are no multiple of 64, and up to 64 rows a call without scratch: refused with a reason, on buffers of the whole
+    size, so that a refusal that got lost would show as a stored output and nothing worse."""
+    from eet_b200 import _lib
+    k, n = (K + 63) // 64 * 64, (N + 63) // 64 * 64
+    x, out = torch.zeros(M, k, dtype=torch.float16, device="cuda"), torch.full((M, n), 7.0, dtype=torch.float16, device="cuda")
+    w, s = torch.zeros(k, n, dtype=torch.int8, device="cuda"), torch.zeros(n, dtype=torch.float16, device="cuda")
+    rc = _lib.lib.eet_gemm_w8a16(x.data_ptr(), w.data_ptr(), s.data_ptr(), out.data_ptr(), M, N, K, None, 0, None, 0,
+                                 torch.cuda.current_stream().cuda_stream)
+    assert rc != 0 and (b"multiples of 64" if (k, n) != (K, N) else b"workspace") in _lib.lib.eet_last_error()
+    assert bool((out == 7.0).all())
+
+
 def test_empty_and_invalid():
     from eet_b200 import EET, _lib
     x, q, s = _case(64, 64, 1)
