@@ -105,6 +105,48 @@ def test_calls_behind_one_another_give_the_same_bits(K, N, M):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("K,N,M", [(4096, 3968, 40), (4096, 3968, 64), (11008, 3968, 17), (11008, 3968, 33), (1984, 8320, 48)])
+def test_stream_k_calls_behind_one_another_give_the_same_bits(K, N, M):
+    """The stream-K kernel with tiles of 32 and of 64 tokens, two CTAs an SM and rings that wrap, on shapes that the tiles with the
+    weights in tensor memory do not take (the plan is part of the case): six hundred calls that nothing waits between, on exact
+    sums, and a scratch that is zero again behind them."""
+    from eet_b200 import EET, _lib
+    assert _plan(M, N, K)[0] == STREAM_K
+    gen = torch.Generator(device="cuda").manual_seed(N + M)
+    q = torch.randint(-127, 128, (K, N), generator=gen, device="cuda", dtype=torch.int8)
+    s = torch.full((N,), 2.0 ** -10, device="cuda").half()
+    x = torch.randint(-4, 5, (M, K), generator=gen, device="cuda").half()
+    packed = EET.preprocess_weights(q)
+    want = ((x.double() @ q.double()) * 2.0 ** -10).half()
+    outs = torch.empty(50, M, N, dtype=torch.float16, device="cuda")
+    for _ in range(12):
+        for out in outs:
+            EET.gemm_w8a16(x, packed, s, out=out)
+        assert bool((outs == want).all())
+    assert all(int(ws.view(torch.int32).abs().max()) == 0 for ws in EET._pool.gemm_ws.values())
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("K,N,M,two", [(4096, 11008, 32, True), (4096, 11008, 64, True), (11008, 4096, 17, False), (4096, 12288, 64, False)])
+def test_stream_k_sums_behind_one_another_are_exact(K, N, M, two):
+    """eet_gemm_w8a16_accum as a decode chain of 17 to 64 rows calls it (gate and up in one launch, down, QKV), which takes the
+    stream-K kernel whatever the dispatch gives a plain call: six hundred launches that nothing waits between.  Whole numbers:
+    twelve products on top of one another stay below 2^24, so every sum is exact whatever the order."""
+    from eet_b200 import EET, _lib
+    gen = torch.Generator(device="cuda").manual_seed(N + M)
+    x = torch.randint(-4, 5, (M, K), generator=gen, device="cuda").half()
+    q = [torch.randint(-127, 128, (K, N), generator=gen, device="cuda", dtype=torch.int8) for _ in range(2 if two else 1)]
+    packed = [EET.preprocess_weights(w) for w in q]
+    want = [x.double() @ w.double() for w in q]
+    assert all(float(w.abs().max()) * 12 < 2 ** 24 for w in want)
+    sums = [torch.zeros(50, M, N, device="cuda") for _ in q]
+    for rep in range(1, 13):
+        for i in range(50):
+            EET.gemm_w8a16_accum(x, packed[0], sums[0][i], *((packed[1], sums[1][i]) if two else ()))
+        assert all(bool((t.double() == rep * w).all()) for t, w in zip(sums, want))
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("epilogue", ["plain", "residual"])
 @pytest.mark.parametrize("n,M", [(4096, 3), (4096, 16), (1024, 8), (192, 9), (4096, 40), (4096, 100), (4096, 200), (192, 300)])
 def test_output_over_the_activations(n, M, epilogue):
