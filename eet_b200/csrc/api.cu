@@ -226,7 +226,11 @@ struct GemmRoute {
 // models are off by 6 to 8 %: nearer than that the measured times were equal or the other way round (5120 x 13696, M = 1024:
 // modelled 106 us, measured 120, tiles with the weights in shared memory 114).  Stream-K has become a tenth faster than its
 // model since that was fitted (4096 x 4096, M = 100: 12.3 us, modelled 13.9, these tiles 11.2; M = 160: 17.2 and 12.6).
-constexpr double kTsMargin = 0.85, kTsMarginStreamK = 0.78;
+// Up to 64 rows the only other is stream-K, which wins where the tiles leave many SMs idle in a wave (8192 x 19200, M = 17:
+// stream-K 34.8 us, 75 tiles 39.7) or just begin another (5120 x 38016, M = 17: 42.5, 149 tiles 52 to 67).  With these models 5
+// of 1614 measured calls are more than 2 % slower than on stream-K as it was without the tiles, 4 % at most, and none that
+// the tiles made faster has lost more than that but two.
+constexpr double kTsMargin = 0.85, kTsMarginStreamK = 0.78, kTsMarginFewRows = 1.04;
 
 static GemmRoute gemm_route(int M, int N, int K, bool scratch)
 {
@@ -251,7 +255,7 @@ static GemmRoute gemm_route(int M, int N, int K, bool scratch)
         least = r.pair.us;
     }
     const Tc2Plan ts = gemm_ts_plan(M, N, K);
-    if (ts.us < (M < kTcMinM ? 1e30 : (r.kernel == kRouteStreamK ? kTsMarginStreamK : kTsMargin) * least)) {
+    if (ts.bn > 0 && ts.us < (M < kTcMinM ? kTsMarginFewRows : (r.kernel == kRouteStreamK ? kTsMarginStreamK : kTsMargin)) * least) {
         r.kernel = kRouteTiles;
         r.ts = true;
         r.tc = ts;

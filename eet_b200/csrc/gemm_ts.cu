@@ -687,6 +687,10 @@ Tc2Plan gemm_ts_plan(int M, int N, int K)
             double us = (units + S - 1) / S * unit * (block > reading ? block : reading) + 2.86 + 0.0214 * bn;
             if (S > 1) us += 1.13 + 0.0145 * ((chunks + S - 1) / S * (S - 1) * chunk) + (tiles_m > 1 ? 0.9 : 0.0);
             us = rounds * us - 0.34;
+            // Up to 64 rows: CTAs without a second tile leave HBM to the others and their SM to the next kernel (149 to 400
+            // tiles, measured 0.68 to 0.90 of full rounds); clusters of five to eight that end at different times do not
+            // find room again at once (4 to 25 % longer).
+            if (rounds > 1 && M < kTcMinM) us *= S == 1 ? 0.85 : (S > 4 ? 1.1 : 1.0);
             if (us < best.us) best = Tc2Plan{bn, (int)tiles, S == 1 ? (int)tiles : 0, S, us};
         }
     }

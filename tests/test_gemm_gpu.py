@@ -343,6 +343,29 @@ def test_tiles_with_the_weights_in_tensor_memory(K, N, M, bn, split, tiles, kind
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("K,N,M,kernel,tiles", [
+    (8192, 19200, 17, STREAM_K, 0), (12160, 19968, 23, STREAM_K, 0), (16384, 19968, 17, STREAM_K, 0), (5120, 38016, 17, STREAM_K, 0),
+    (4096, 38016, 32, STREAM_K, 0), (8192, 19200, 48, TILES, 75), (8192, 22016, 48, TILES, 86), (8192, 24576, 17, TILES, 96),
+    (2048, 38016, 64, TILES, 149), (4096, 51200, 40, TILES, 200), (4096, 64000, 32, TILES, 250)])
+def test_wide_matrices_of_17_to_64_rows_take_the_faster_kernel(K, N, M, kernel, tiles):
+    """Tiles that would leave many SMs idle, or begin another wave for a few, against stream-K (measured, us: 8192 x 19200, M = 17,
+    stream-K 35, tiles 40; 12160 x 19968, M = 23, 51 and 65; 5120 x 38016, M = 17, 43 and 52 to 67; the other way round 8192 x
+    22016, M = 48, 47 and 39; 2048 x 38016, M = 64, 29 and 22; 4096 x 64000, M = 32, 66 and 52).  And right: one rounding to fp16,
+    doubled."""
+    from eet_b200 import EET, _lib
+    assert _plan(M, N, K)[0] == kernel and (kernel == STREAM_K or _plan(M, N, K)[2:] == (tiles, 0, 1))
+    assert _lib.lib.eet_gemm_w8a16_weights_in_tmem(M, N, K) == (kernel == TILES)
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    q = torch.randint(-127, 128, (K, N), generator=gen, device="cuda", dtype=torch.int8)
+    s = ((torch.rand(N, generator=gen, device="cuda") + 0.5) * K ** -0.5 / 64).half()
+    x = torch.randn(M, K, generator=gen, device="cuda").half()
+    out = EET.gemm_w8a16(x, EET.preprocess_weights(q), s)
+    for c in range(0, N, 8192):
+        y = (x.double() @ q[:, c:c + 8192].double()) * s[c:c + 8192].double()
+        assert ((out[:, c:c + 8192].double() - y).abs() <= 2.0 ** -10 * y.abs() + 1e-4).all()
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("K,N,M,taken", [
     (4096, 4096, 16, 0), (4096, 4096, 17, 1), (4096, 3968, 40, 0), (1984, 4096, 40, 0), (4096, 4224, 40, 0), (4096, 8320, 40, 1),
     (4096, 4096, 64, 1), (4096, 4096, 100, 0), (4096, 11008, 100, 1), (13696, 5120, 999, 1), (5120, 13696, 999, 0), (4096, 4096, 4096, 0)])
