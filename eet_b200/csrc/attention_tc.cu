@@ -162,12 +162,6 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&v)[kPtK])
 }
 
 // The FP32 operations of the softmax, two scores at a time (one instruction for a pair of registers).
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
-{
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
 {
     uint64_t d;

@@ -24,8 +24,6 @@
 // Not taken: three sets of conversion warps (instruction issue is what they share: 850 cycles a k-block); one set and two CTAs per SM
 // (4096 x 11008, M = 32: 14.9 us, 13.0 here); partial sums through the copy engine (16.9 us at M = 100, 16.5 as they are).
 // Every wait is bounded (device status 2), tensor memory is freed on every path, and the CTAs of a cluster end together.
-#include <cooperative_groups.h>
-
 #include "common.cuh"
 #include "kernels.h"
 
