@@ -209,9 +209,10 @@ int eet_gemm_w8a16_finalize(float* sums, const void* scale, const void* residual
 // Which kernel a shape goes to.  Up to 16 rows the row kernel, or equal shares with a finishing launch.  Above that tiles with the
 // weights in tensor memory (N and K large enough to have been measured), stream-K units into fp32 scratch with a finishing
 // launch, tiles with the weights in shared memory or tiles on CTA pairs, all but the units with the epilogue fused: the shortest
-// modelled time decides, among those that the shape may take; up to 64 rows it is the first kind, where it takes the shape
-// (4096 x 12288, M = 64: 14.9 us, stream-K 20.2; 11008 x 4096, M = 32: 14.2 and 13.9).  Measured on both sides of the lines: 4096 x 4096, M = 128 units 15 us, tiles 18, and at M = 256
-// 21.7 and 20.2; 4096 x 32000, M = 384 units 148, tiles 100, pairs 94; 11008 x 4096, M = 4096 single CTAs 267, pairs 249.
+// modelled time decides, among those that the shape may take (up to 64 rows only the first two are).  Measured on both sides of
+// the lines, in a chain of calls, us (weights in tensor memory / stream-K / tiles / pairs): 4096 x 12288, M = 64 15.0 / 18.9;
+// 11008 x 4096, M = 32 14.7 / 14.2; 4096 x 4096, M = 128 11.7 / 13.5 / 16.7, M = 256 15.4 / 19.1 / 19.4 / 32.3; 4096 x 1536, M = 512
+// - / 15.5 / 18.5 / 32.3; 4096 x 32000, M = 384 79.1 / 146 / 96.6 / 81.0; 11008 x 4096, M = 4096 - / - / 278 / 246.
 enum { kRouteShares = 0, kRouteRow = 1, kRouteStreamK = 2, kRouteTiles = 3, kRoutePairs = 4 };
 
 struct GemmRoute {
@@ -223,9 +224,10 @@ struct GemmRoute {
 };
 
 // Above 64 rows the tiles with the weights in tensor memory must be modelled this much shorter than the best of the others, whose
-// models are off by 6 to 8 %: nearer than that the measured times were equal or the other way round (5120 x 13696, M = 1024:
-// modelled 106 us, measured 120, tiles with the weights in shared memory 114).  Stream-K has become a tenth faster than its
-// model since that was fitted (4096 x 4096, M = 100: 12.3 us, modelled 13.9, these tiles 11.2; M = 160: 17.2 and 12.6).
+// models were fitted before their single threads were chosen by elect.sync: stream-K measures up to 11 % less than modelled
+// (4096 x 4096: M = 100 12.7 us, modelled 13.9; M = 160 17.3 and 19.2), tiles with the weights in shared memory up to 20 %
+// (5120 x 13696, M = 256: 37.7 and 45.6).  The margins keep what is not certain on the others' side, also where these tiles
+// measure less: 4096 x 4096 at M = 100 11.4 (modelled 11.1), 8192 x 22016 at M = 384 113 (111), tiles in shared memory 136 (129).
 // Up to 64 rows the only other is stream-K, which wins where the tiles leave many SMs idle in a wave (8192 x 19200, M = 17:
 // stream-K 34.8 us, 75 tiles 39.7) or just begin another (5120 x 38016, M = 17: 42.5, 149 tiles 52 to 67).  With these models 5
 // of 1614 measured calls are more than 2 % slower than on stream-K as it was without the tiles, 4 % at most, and none that

@@ -24,7 +24,8 @@
 //                      SCORE COLUMNS as fp16 pairs (tcgen05.st: a row only ever touches its own lane, and the
 //                      tensor core overwrites a score buffer only after the P.V that read it, in issue order);
 //                      the O accumulator is rescaled only when a row's maximum has outgrown the one that O is
-//                      accumulated under by 2^8.  At the end they read O, normalise and store the context.
+//                      accumulated under by 2^8 (the conditional rescaling that FlashAttention-4 made known).  At the
+//                      end they read O, normalise and store the context.
 // Every wait is bounded (device status 2) and the CTA frees its tensor memory on every path.
 //
 // Numerics kept from the reference and from the mma.sync kernel this one replaces for long prompts: scores scaled
@@ -32,8 +33,8 @@
 // above the left padding are zero.  The scores stay in fp32: the reference stores them as fp16, which costs more than half of
 // the error of the result (relative to 64 bits 4.4e-4 with that rounding, 2.6e-4 without it, 2 x 2048 tokens).
 //
-// Measured, 32 heads: 2 x 2048 tokens 89 us (138 with a rescale of O in nearly every block, one chain of 64 maxima, the
-// tiles of a pair behind one another and the fp16 rounding), 8 x 512 48 us (58); 40 heads with a bias, 2 x 701 tokens 41 us
+// Measured, 32 heads: 2 x 2048 tokens 85 us (136 with a rescale of O in nearly every block, one chain of 64 maxima, the
+// tiles of a pair behind one another and the fp16 rounding), 8 x 512 46 us (57); 40 heads with a bias, 2 x 701 tokens 40 us
 // (56).  Time stamps: a block takes 1650 cycles on each of an SM's two CTAs, and the issuing thread is the one that never waits: Q.K^T
 // with 64 keys reads 6 KiB of shared memory per MMA (48 cycles) for 32 cycles of multiplications.
 #include <cuda.h>
@@ -521,7 +522,7 @@ bool prefill_mha_tc_supported(int S, int D)
 int launch_prefill_mha_tc(const __half* q, const __half* kcache, const __half* vcache, __half* ctx, int B, int S, int H,
                           int T_max, const int64_t* pad_len, const __half* alibi, int alibi_stride, cudaStream_t stream)
 {
-    EET_CHECK((long long)B * H <= 65535, "prefill attention: batch x heads = %lld exceeds the grid limit", (long long)B * H);
+    EET_CHECK((long long)B * H <= 65535, "prefill attention: batch x heads = %lld exceeds 65535", (long long)B * H);
     CUtensorMap map_q, map_k, map_v;
     if (int rc = encode_rows_map(&map_q, q, S, (size_t)S, B * H, kPtQ)) return rc;
     if (int rc = encode_rows_map(&map_k, kcache, S, (size_t)T_max, B * H, kPtK)) return rc;

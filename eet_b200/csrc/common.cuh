@@ -65,9 +65,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p)
 }
 
 // True for one lane of the (whole) warp, always the same one.  The roles that issue TMA copies and tcgen05 instructions are one
-// thread, and it is chosen with this and not with lane == 0: these instructions take their operands from uniform registers, and
-// only behind elect.sync does the compiler know that a single thread is active.  Behind lane == 0 it serialises over the lanes
-// that might be: eight MMAs and two commits took 750 to 950 cycles to issue, against 130 to 170 behind this.
+// thread, and it is chosen with this and not with lane == 0.  Measured: eight MMAs and two commits take 130 to 170 cycles to issue
+// behind this, 750 to 950 behind lane == 0.  (Presumably because only elect.sync tells the compiler that one thread is active.)
 __device__ __forceinline__ bool elect_one()
 {
     uint32_t pred;

@@ -447,7 +447,8 @@ static int mid_bn(int M, long long units)
 
 // Modelled time with the finishing launch, above 64 rows: per token tile and unit per SM 0.65 us at 128 tokens and 0.86 at 256, and
 // 3.4 ps for each fp32 sum that goes to memory and back.  Fitted to 190 measured times at 65 to 512 rows on 16 weight shapes
-// from 4096 x 1536 to 8192 x 24576, spread 3 %.
+// from 4096 x 1536 to 8192 x 24576, spread 3 %, before the issuing threads were chosen by elect.sync; calls of 12 to 180 us have
+// since measured 11 % less to 8 % more than this (4096 x 4096, M = 100: 12.7 for 13.9; 8192 x 22016, M = 384: 182 for 168).
 // Up to 64 rows, where a unit is bound by HBM: 0.45 us, with tiles of 64 tokens 0.53.  Fitted to 1614 measured calls on 4096 to
 // 102400 channels, reductions of 2048 to 22016, spread 6 %.
 double gemm_mid_us(int M, int N, int K)

@@ -14,8 +14,8 @@
 // The barriers between the two CTAs use the default (CTA) scope: what they guard is read and written by the tensor cores and
 // the TMA engine, ordered by the proxy fence and the tensor-memory fences beside them.  With cluster-scope acquire in the
 // waits a k-block took 1.25 us instead of 0.66, whatever the depth of the rings.
-// Measured (a call, one-CTA kernel in brackets): 11008 x 4096 at M = 4096 246 us = 1.50 PF/s (288), at M = 2048 125 (141),
-// 5120 x 13696 at M = 4096 400 (432), 4096 x 11008 at M = 2048 134 (147; 160 before its single threads were chosen by elect.sync).
+// Measured (a call, one-CTA kernel in brackets): 11008 x 4096 at M = 4096 246 us = 1.50 PF/s (278), at M = 2048 125 (137),
+// 5120 x 13696 at M = 4096 398 (429), 4096 x 11008 at M = 2048 133 (148).
 // Every wait is bounded (device status 2), tensor memory is freed on every path.
 #include "common.cuh"
 #include "kernels.h"
@@ -390,8 +390,10 @@ PairPlan gemm_pair_plan(int M, int N, int K)
     for (int bn = 256; bn >= 128; bn -= 16) {
         const long long tiles = (long long)tiles_n * ((M + 2 * bn - 1) / (2 * bn));
         if (tiles > 0x3fffffffLL) continue;
-        // a k-block with the machine full: fitted to 110 calls of 256 to 4096 rows at K from 4096 on; below, where a tile's start and
-        // end weigh as much, as measured before its threads were chosen by elect.sync
+        // a k-block with the machine full: fitted to 110 calls of 256 to 4096 rows at K from 4096 on, the smallest that was measured;
+        // below, the constants from before the single threads were chosen by elect.sync.  Those are too long by 13 to 24 % (1024
+        // x 4096 at M = 1024: 13.8 us for 18.1; 3072 x 8192 at M = 2048: 78 for 90), as the one-CTA kernel's are by 3 to 18 %
+        // (15.1 for 18.2; 83 for 88)
         const double block = K >= 4096 ? 0.60 + 0.0018 * (bn - 192) : 0.65 + 0.00203 * (bn - 192);
         const double us = 7.0 + (double)((tiles + pairs - 1) / pairs) * (KT * block + 1.5 + 0.01 * bn);
         if (us < best.us) best = PairPlan{bn, us};

@@ -728,9 +728,11 @@ static double tc2_block_us(int bn)
 
 // The plan with the least modelled time over all BN and ways to treat the tiles that fill no wave.  A launch costs 5.5 us
 // around its tiles, a tile's epilogue is not overlapped with its CTA's next tile, a cluster pays for two barriers and the
-// exchange of partial sums, a second launch for its start.  Against measurements at M = 100 ... 4096 on the LLaMA-7B and
-// Baichuan-13B shapes the model is within 10 %; it knows no power limit, which makes calls of milliseconds longer by up to a
-// sixth (8192 x 22016 at M = 8192: 2.0 ms here, 2.3 measured) whatever the plan.
+// exchange of partial sums, a second launch for its start.  When it was fitted, at M = 100 ... 4096 on the LLaMA-7B and
+// Baichuan-13B shapes, the model was within 10 %; since the issuing thread is chosen by elect.sync calls below 50 us measure up to
+// a fifth less (4096 x 4096, M = 100: 16.6 us for 20.9; 5120 x 13696, M = 256: 37.7 for 45.6; 11008 x 4096, M = 4096: 278 for 280).
+// It knows no power limit, which makes calls of milliseconds longer by up to a sixth (8192 x 22016 at M = 8192: 2.0 ms here, 2.3
+// measured) whatever the plan.
 static Tc2Plan tc2_plan(int M, int N, int K)
 {
     const int KT = K / kTile, G = sm_count();

@@ -109,9 +109,9 @@ size_t eet_gemm_w8a16_workspace_bytes(int M, int N, int K);
  * M may be any value >= 0; K and N must be multiples of 64; pointers 16-byte aligned.  C may lie over A up to 64 rows, and up
  * to 512 for narrow shapes (below), with scratch.
  * Kernels: M <= 16 the row kernel (one launch, leaves the scratch alone), wide matrices that would leave its last wave
- * mostly empty the equal-share kernel into the scratch with a finishing launch; 16 < M <= 64 (N % 128 == 0) tiles of 256
- * channels with the weights in tensor memory (N >= 4096, K >= 2048) or stream-K into the scratch with a finishing launch;
- * above that the shortest modelled time decides between these, tiles with the weights in shared memory, both on single CTAs
+ * mostly empty the equal-share kernel into the scratch with a finishing launch; above that (N % 128 == 0) the shortest
+ * modelled time decides: 16 < M <= 64 between tiles of 256 channels with the weights in tensor memory (N >= 4096, K >= 2048)
+ * and stream-K into the scratch with a finishing launch; from 65 rows also tiles with the weights in shared memory, both on single CTAs
  * or with the reduction split over clusters of 2-8, and tiles on CTA pairs (from 256 rows); shapes with N % 128 == 64 take
  * the equal-share kernel in groups of 128 rows.
  * Scratch is needed for M <= 64, for N % 128 == 64, and for C over A.  Up to 512 rows, narrow shapes (N % 256 != 0, or
